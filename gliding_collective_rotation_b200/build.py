@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -38,14 +39,16 @@ def build(verbose=False, force=False):
         return LIB
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
-    objs = []
-    for s in srcs:
-        o = os.path.join(objdir, os.path.basename(s).replace(".cu", ".o"))
-        cmd = [nvcc(), *ARCH, *FLAGS, "-c", s, "-o", o]
+    objs = [os.path.join(objdir, os.path.basename(s).replace(".cu", ".o")) for s in srcs]
+
+    def compile_one(src, obj):
+        cmd = [nvcc(), *ARCH, *FLAGS, "-c", src, "-o", obj]
         if verbose:
             cmd += ["-Xptxas", "-v"]
         subprocess.run(cmd, check=True)
-        objs.append(o)
+
+    with ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        list(pool.map(compile_one, srcs, objs))
     tmp = LIB + ".tmp"
     subprocess.run([nvcc(), *ARCH, "-shared", "-o", tmp, *objs, "-lcudart"], check=True)
     os.replace(tmp, LIB)

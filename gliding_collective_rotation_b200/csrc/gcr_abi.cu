@@ -132,8 +132,7 @@ struct gcr_ctx {
     int *d_row_prefix = nullptr;  // row tiles of the cell-staged pair kernel per slot, prefix [S + 1]
     int *d_ntiles = nullptr;  // [0] bead tiles, [1] cell tiles
     uint8_t *topo = nullptr;
-    int *cnt = nullptr;
-    int *ncell = nullptr;
+    int *cnt[2] = {nullptr, nullptr};  // beads per cell, in turns (SysS::turn)
     int *items = nullptr;
     int *nbr = nullptr;
     int *ncount = nullptr;
@@ -145,9 +144,10 @@ struct gcr_ctx {
     void *fp = nullptr;
     double *pos2 = nullptr;  // SRK4 scratch: second virtual update
     void *faux = nullptr;    // SRK4 scratch: stage forces of systems without a caller buffer
-    size_t stage_smem = 0;
     size_t pair_cells_smem = 0;
     size_t pair_smem = 0;
+    size_t stage_smem = 0;
+    size_t build_smem = 0;
     int32_t *chain_starts = nullptr;
     int *d_err = nullptr;
     double *d_out = nullptr;
@@ -181,6 +181,10 @@ struct gcr_ctx {
 };
 
 namespace {
+
+// list entries a thread of the list build sorts in shared memory, of which it
+// takes from the L1 cache: short lists (WCA) need few
+int build_cap(int block, int list_depth) { return std::min(list_depth <= 32 ? 12 : 32, 12288 / block); }
 
 int kernel_grid(const gcr_ctx *c, void *fn, int block, int64_t max_tiles, size_t smem = 0)
 {
@@ -541,25 +545,23 @@ int launch(gcr_ctx *c, void *fn, int grid, int block, size_t smem = 0)
     return launch_args(c, fn, grid, block, smem, a);
 }
 
-int launch_sys(gcr_ctx *c, void *fn)
+// the per-system work between two kernels of a step (kDuty...)
+int launch_duty(gcr_ctx *c, int duty)
 {
-    int n = (int)c->slots.size();
-    void *a[] = {&c->args, &n};
-    return launch_args(c, fn, c->grid_sys, 128, 0, a);
+    void *a[] = {&c->args, &duty};
+    return launch_args(c, c->ks.duty, 1, 1024, 0, a);
 }
 
-// one stage's neighbour lists (flagged systems only): plan, bin, per-cell
-// sort, build
+// one stage's neighbour lists, of the systems that the plan took: bin, (for the cell-staged pair forces) per-cell sort, build
 int enqueue_lists(gcr_ctx *c, int which)
 {
     int rc;
-    const int bb = c->cfg.block_beads, bc = c->cfg.block_cells;
+    const int bb = c->cfg.block_beads;
     void *bin = which == 0 ? c->ks.bin0 : (which == 1 ? c->ks.bin1 : c->ks.bin2);
     void *build = which == 0 ? c->ks.build0 : (which == 1 ? c->ks.build1 : c->ks.build2);
-    if ((rc = launch(c, c->ks.lists_plan, 1, 1024))) return rc;
     if ((rc = launch(c, bin, c->grid_bin, bb))) return rc;
-    if ((rc = launch(c, c->ks.sort, c->grid_sort, bc))) return rc;
-    return launch(c, build, c->grid_build, bb);
+    if (c->cfg.pair_mode == 2 && (rc = launch(c, c->ks.sort, c->grid_sort, c->cfg.block_cells))) return rc;
+    return launch(c, build, c->grid_build, bb, c->build_smem);
 }
 
 // the in-graph order-parameter series: one 1024-thread CTA per slot
@@ -584,11 +586,11 @@ int enqueue_step4(gcr_ctx *c)
         if ((rc = launch(c, pair, c->grid_pair, bb, c->pair_smem))) return rc;
         if ((rc = launch(c, c->ks.stage4[k], c->grid_stage4[k], bb, c->stage_smem))) return rc;
         if (k < 3 && c->graph_rigid && (rc = launch(c, c->ks.rigid4[k], c->grid_update, bb))) return rc;
+        if ((rc = launch_duty(c, k < 3 ? kDutyPlan : kDutyDt))) return rc;
     }
-    if ((rc = launch_sys(c, c->ks.sys_dt))) return rc;
     if ((rc = launch(c, c->ks.update, c->grid_update, bb))) return rc;
     if (c->graph_rigid && (rc = launch(c, c->ks.rigid4[3], c->grid_update, bb))) return rc;
-    if ((rc = launch_sys(c, c->ks.sys_end))) return rc;
+    if ((rc = launch_duty(c, kDutyEnd))) return rc;
     return c->graph_obs ? launch_observe(c) : GCR_OK;
 }
 
@@ -600,19 +602,32 @@ bool fused_pair(const gcr_ctx *c, bool cross) { return pair_mode(c, cross) == 1;
 // SRK2 stage s (0 predictor, 1 corrector): the pair forces, then the stage
 int enqueue_pair(gcr_ctx *c, int s, bool cross)
 {
-    const int mode = pair_mode(c, cross);
-    if (mode == 1) return GCR_OK;
-    if (mode == 2) return launch(c, c->ks.pair_cells[s], c->grid_pair_cells, c->cfg.block_beads, c->pair_cells_smem);
+    if (fused_pair(c, cross)) return GCR_OK;
+    if (pair_mode(c, cross) == 2) return launch(c, c->ks.pair_cells[s], c->grid_pair_cells, c->cfg.block_beads, c->pair_cells_smem);
     void *pair = cross ? c->ks.pair_cross[s] : (s == 0 ? c->ks.pair0 : c->ks.pair1);
     return launch(c, pair, c->grid_pair, c->cfg.block_beads, c->pair_smem);
 }
 
-int enqueue_stage(gcr_ctx *c, int s, bool cross)
+// the stage; the dt rule after the corrector, the list plan of the corrector
+// after the predictor
+int enqueue_stage(gcr_ctx *c, int s, bool cross, bool rigid)
 {
     const bool f = fused_pair(c, cross);
     void *stage = s == 0 ? (f ? c->ks.stage0f : c->ks.stage0) : (f ? c->ks.stage1f : c->ks.stage1);
     const int grid = s == 0 ? (f ? c->grid_stage0f : c->grid_stage0) : (f ? c->grid_stage1f : c->grid_stage1);
-    return launch(c, stage, grid, c->cfg.block_beads, c->stage_smem);
+    const int bb = c->cfg.block_beads;
+    int rc = launch(c, stage, grid, bb, c->stage_smem);
+    if (!rc && s == 0 && rigid) rc = launch(c, c->ks.rigid0, c->grid_update, bb);
+    return rc ? rc : launch_duty(c, s == 0 ? kDutyPlan : kDutyDt);
+}
+
+// the corrector's update, and the step's bookkeeping
+int enqueue_update(gcr_ctx *c, bool rigid)
+{
+    const int bb = c->cfg.block_beads;
+    int rc = launch(c, c->ks.update, c->grid_update, bb);
+    if (!rc && rigid) rc = launch(c, c->ks.rigid1, c->grid_update, bb);
+    return rc ? rc : launch_duty(c, kDutyEnd);
 }
 
 int enqueue_step(gcr_ctx *c)
@@ -623,16 +638,12 @@ int enqueue_step(gcr_ctx *c)
     if ((rc = enqueue_lists(c, 0))) return rc;
     if ((rc = enqueue_pair(c, 0, c->graph_cross))) return rc;
     if (c->graph_motor && (rc = launch(c, c->ks.motor[0], c->grid_update, bb))) return rc;
-    if ((rc = enqueue_stage(c, 0, c->graph_cross))) return rc;
-    if (c->graph_rigid && (rc = launch(c, c->ks.rigid0, c->grid_update, bb))) return rc;
+    if ((rc = enqueue_stage(c, 0, c->graph_cross, c->graph_rigid))) return rc;
     if ((rc = enqueue_lists(c, 1))) return rc;
     if ((rc = enqueue_pair(c, 1, c->graph_cross))) return rc;
     if (c->graph_motor && (rc = launch(c, c->ks.motor[1], c->grid_update, bb))) return rc;
-    if ((rc = enqueue_stage(c, 1, c->graph_cross))) return rc;
-    if ((rc = launch_sys(c, c->ks.sys_dt))) return rc;
-    if ((rc = launch(c, c->ks.update, c->grid_update, bb))) return rc;
-    if (c->graph_rigid && (rc = launch(c, c->ks.rigid1, c->grid_update, bb))) return rc;
-    if ((rc = launch_sys(c, c->ks.sys_end))) return rc;
+    if ((rc = enqueue_stage(c, 1, c->graph_cross, c->graph_rigid))) return rc;
+    if ((rc = enqueue_update(c, c->graph_rigid))) return rc;
     return c->graph_obs ? launch_observe(c) : GCR_OK;
 }
 
@@ -641,7 +652,8 @@ int enqueue_step(gcr_ctx *c)
 // others keep their lists
 int enqueue_run_start(gcr_ctx *c)
 {
-    return launch(c, c->ks.run_check, c->grid_update, c->cfg.block_beads);
+    int rc = launch(c, c->ks.run_check, c->grid_update, c->cfg.block_beads);
+    return rc ? rc : launch_duty(c, kDutyStart);
 }
 
 // a list build of `slot` before its next pair forces, from zeroed cell
@@ -652,7 +664,8 @@ int mark_rebuild(gcr_ctx *c, int slot)
 {
     const Slot &sl = c->slots[slot];
     if (sl.n_cells_alloc > 0)
-        GCR_CUDA(cudaMemsetAsync(c->cnt + sl.cell_off, 0, sizeof(int) * (size_t)sl.n_cells_alloc, c->stream));
+        for (int *cnt : c->cnt)
+            GCR_CUDA(cudaMemsetAsync(cnt + sl.cell_off, 0, sizeof(int) * (size_t)sl.n_cells_alloc, c->stream));
     int n = (int)c->slots.size();
     void *a[] = {&c->args, &n, &slot};
     GCR_CUDA(cudaLaunchKernel(c->ks.sys_mark, dim3(c->grid_sys), dim3(128), a, 0, c->stream));
@@ -787,8 +800,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     e = e ? e : cudaMalloc(&c->d_row_prefix, sizeof(int) * (size_t)(S + 1));
     e = e ? e : cudaMemsetAsync(c->d_row_prefix, 0, sizeof(int) * (size_t)(S + 1), c->stream);
     e = e ? e : cudaMalloc(&c->topo, (size_t)cfg.bead_capacity);
-    e = e ? e : cudaMalloc(&c->cnt, sizeof(int) * cells_alloc);
-    e = e ? e : cudaMalloc(&c->ncell, sizeof(int) * cells_alloc);
+    for (int k = 0; k < 2; k++) e = e ? e : cudaMalloc(&c->cnt[k], sizeof(int) * cells_alloc);
     e = e ? e : cudaMalloc(&c->items, sizeof(int) * std::max<int64_t>(slots_total, 1));
     e = e ? e : cudaMalloc(&c->nbr, sizeof(int) * (size_t)cfg.bead_capacity * (size_t)cfg.list_depth);
     e = e ? e : cudaMalloc(&c->ncount, sizeof(int) * (size_t)cfg.bead_capacity);
@@ -810,8 +822,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
                             std::string("device allocation: ") + cudaGetErrorString(e)));
     cudaMemsetAsync(c->dS, 0, sizeof(SysS) * S, c->stream);
     cudaMemsetAsync(c->d_ntiles, 0, sizeof(int) * 2, c->stream);
-    cudaMemsetAsync(c->cnt, 0, sizeof(int) * cells_alloc, c->stream);
-    cudaMemsetAsync(c->ncell, 0, sizeof(int) * cells_alloc, c->stream);
+    for (int *cnt : c->cnt) cudaMemsetAsync(cnt, 0, sizeof(int) * cells_alloc, c->stream);
     cudaMemsetAsync(c->ncount, 0, sizeof(int) * (size_t)cfg.bead_capacity, c->stream);
     cudaMemsetAsync(c->img, 0, sizeof(int) * (size_t)cfg.bead_capacity * cfg.dim, c->stream);
     cudaMemsetAsync(c->work, 0, sizeof(int) * (size_t)(3 + 3 * (S + 1)), c->stream);
@@ -829,8 +840,10 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     a.cell_tiles = c->d_cell_tiles;
     a.n_cell_tiles = c->d_ntiles + 1;
     a.topo = c->topo;
-    a.cnt = c->cnt;
-    a.ncell = c->ncell;
+    a.cnt0 = c->cnt[0];
+    a.cnt1 = c->cnt[1];
+    a.build_cap = build_cap(cfg.block_beads, cfg.list_depth);
+    c->build_smem = sizeof(int) * (size_t)a.build_cap * cfg.block_beads;
     a.items = c->items;
     a.nbr = c->nbr;
     a.ncount = c->ncount;
@@ -883,7 +896,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     c->grid_pair = kernel_grid(c, c->ks.pair0, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
     c->grid_bin = kernel_grid(c, c->ks.bin0, cfg.block_beads, c->max_bead_tiles);
     c->grid_sort = kernel_grid(c, c->ks.sort, cfg.block_cells, c->max_cell_tiles);
-    c->grid_build = kernel_grid(c, c->ks.build0, cfg.block_beads, c->max_bead_tiles);
+    c->grid_build = kernel_grid(c, c->ks.build0, cfg.block_beads, c->max_bead_tiles, c->build_smem);
     c->grid_sys = (int)((S + 127) / 128);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return cleanup(fail(GCR_ERR_CUDA, "initialisation"));
     *out = c;
@@ -895,9 +908,8 @@ int gcr_destroy(gcr_ctx *c)
     if (!c) return GCR_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->graph) cudaGraphExecDestroy(c->graph);
-    void *ptrs[] = {c->dP, c->dS, c->d_bead_tiles, c->d_cell_tiles, c->d_ntiles, c->d_row_prefix, c->topo, c->cnt,
-                    c->ncell,
-                    c->items, c->nbr, c->ncount, c->xref, c->work, c->xi, c->fp, c->chain_starts, c->d_err,
+    void *ptrs[] = {c->dP, c->dS, c->d_bead_tiles, c->d_cell_tiles, c->d_ntiles, c->d_row_prefix, c->topo, c->cnt[0],
+                    c->cnt[1], c->items, c->nbr, c->ncount, c->xref, c->work, c->xi, c->fp, c->chain_starts, c->d_err,
                     c->d_out, c->pos2, c->faux, c->xnbr, c->xcount, c->img, c->act, c->mpush, c->mdelta, c->restb};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -1368,20 +1380,16 @@ int gcr_profile_steps(gcr_ctx *c, int32_t n_steps, float *ms_out)
         if (!rc) rc = enqueue_pair(c, 0, cross);  // nothing with fused stages
         if (!rc && any_motor(c)) rc = launch(c, c->ks.motor[0], c->grid_update, bb);
         GCR_CUDA(cudaEventRecord(e[2], c->stream));
-        if (!rc) rc = enqueue_stage(c, 0, cross);
-        if (!rc && rigid) rc = launch(c, c->ks.rigid0, c->grid_update, bb);
+        if (!rc) rc = enqueue_stage(c, 0, cross, rigid);
         GCR_CUDA(cudaEventRecord(e[3], c->stream));
         if (!rc) rc = enqueue_lists(c, 1);
         GCR_CUDA(cudaEventRecord(e[4], c->stream));
         if (!rc) rc = enqueue_pair(c, 1, cross);
         if (!rc && any_motor(c)) rc = launch(c, c->ks.motor[1], c->grid_update, bb);
         GCR_CUDA(cudaEventRecord(e[5], c->stream));
-        if (!rc) rc = enqueue_stage(c, 1, cross);
-        if (!rc) rc = launch_sys(c, c->ks.sys_dt);
+        if (!rc) rc = enqueue_stage(c, 1, cross, rigid);
         GCR_CUDA(cudaEventRecord(e[6], c->stream));
-        if (!rc) rc = launch(c, c->ks.update, c->grid_update, bb);
-        if (!rc && rigid) rc = launch(c, c->ks.rigid1, c->grid_update, bb);
-        if (!rc) rc = launch_sys(c, c->ks.sys_end);
+        if (!rc) rc = enqueue_update(c, rigid);
         GCR_CUDA(cudaEventRecord(e[7], c->stream));
     }
     GCR_CUDA(cudaStreamSynchronize(c->stream));

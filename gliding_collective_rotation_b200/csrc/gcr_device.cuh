@@ -5,9 +5,8 @@
 //     [n,d], chain_id int32 [n], rest_lengths FP64 [n_chains];
 //   * library scratch, per system at a bead / cell offset:
 //       topo      uint8 [bead]        chain-neighbour bits of each bead
-//       cnt       int32 [cell]        beads binned per GPU cell (zeroed by the sort)
-//       ncell     int32 [cell]        beads of each cell at the last list build
-//       items     int32 [cell*depth]  bead ids per cell, sorted by id
+//       cnt0/cnt1 int32 [cell]        beads binned per GPU cell, in turns
+//       items     int32 [cell*depth]  bead ids per cell
 //       nbr       int32 [slot][bead]  neighbour list, slot-major (coalesced
 //                                     across the beads of a warp)
 //       ncount    int32 [bead]        neighbours of each bead
@@ -15,10 +14,10 @@
 //       fp, xi    FT [bead][d]        pair force and step noise per bead
 //   * SysP (read-only during a step) and SysS (device-updated) per slot.
 // Binning writes a fixed-depth table (a count and `depth` slots per cell, the
-// shape of the reference's grid_list, updates.py:502-522); a per-cell sort
-// makes the slot order deterministic; the list build walks the 3^d cells
-// around each bead (the reference's update_nbor_list, updates.py:586-669,
-// with a skin added to the cutoff).
+// shape of the reference's grid_list, updates.py:502-522); the list build
+// walks the 3^d cells around each bead (the reference's update_nbor_list,
+// updates.py:586-669, with a skin added to the cutoff) and sorts each list by
+// id, so the order of the slots does not matter.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -128,7 +127,7 @@ struct SysS {
     int32_t active;
     int32_t flags;
     int32_t rebuild;      // the neighbour list must be rebuilt before the next pair kernel
-    int32_t pad0;
+    int32_t turn;         // list builds planned: which of the two cell counts its cells use
     int64_t list_builds;  // neighbour-list builds since admission
     double *series;       // order-parameter rows of the call (step, elapsed, P, S, angle) or nullptr
     int64_t series_every;

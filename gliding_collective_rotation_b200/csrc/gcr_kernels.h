@@ -17,8 +17,8 @@ struct BatchArgs {
     const Tile *cell_tiles;
     const int *n_cell_tiles;
     const uint8_t *topo;
-    int *cnt;      // beads binned per cell (the sort reads and zeroes it)
-    int *ncell;    // beads per cell at the last list build
+    int *cnt0;     // beads per cell: of a system's last list build in one of the two (SysS::turn),
+    int *cnt1;     // zeroed for its next one in the other
     int *items;    // bead ids per cell, `depth` slots per cell
     int *nbr;      // neighbour list: slot k of bead g at nbr[k * list_stride + g]
     int *ncount;   // neighbours per bead
@@ -26,6 +26,7 @@ struct BatchArgs {
     void *xi;      // translational noise of the current step per bead, FT [bead][dim]
     void *fp;      // pair force per bead (bead order), FT [bead][dim]
     int *work;     // flagged systems of the coming list build (k_lists_plan)
+    int build_cap; // list entries a thread of the build sorts in shared memory
     int n_slots;
     int64_t list_stride;
     int list_depth;
@@ -61,10 +62,13 @@ struct BatchArgs {
     double *restb;
 };
 
+// per-system work after a kernel or phase of the step (gcr_phases.cuh)
+enum { kDutyNone, kDutyStart, kDutyPlan, kDutyDt, kDutyEnd };
+
 struct KernelSet {
     void *bin0;     // cell binning of pos / pos1 for a list build
     void *bin1;
-    void *sort;     // per-cell sort of the binned ids (zeroes the counts)
+    void *sort;     // per-cell sort of the binned ids (cell-staged pair forces)
     void *build0;   // neighbour lists from pos / pos1
     void *build1;
     void *pair0;    // pair forces at pos / pos1
@@ -83,11 +87,9 @@ struct KernelSet {
     void *stage4[4];
     void *rigid4[4];
     void *topo;
-    void *sys_dt;
-    void *sys_end;
+    void *duty;      // per-system work between two kernels of a step (kDuty...), one CTA
     void *sys_mark;  // flag one resident system (or all) for a list build
     void *run_check;  // run start: flag the armed systems whose lists no longer cover their positions
-    void *lists_plan;  // compact the systems that take part in a list build
     void *pair_cross[3];  // pair forces at pos / pos1 / pos2 with the other populations' (coupled systems)
     void *pair_cells[2];  // cell-staged pair forces at pos / pos1 (pair_mode 2)
     void *motor[2];       // motor decisions of stage 0 / 1 (graphs with a motor population)
