@@ -146,7 +146,6 @@ struct gcr_ctx {
     void *faux = nullptr;    // SRK4 scratch: stage forces of systems without a caller buffer
     size_t pair_cells_smem = 0;
     size_t pair_smem = 0;
-    size_t stage_smem = 0;
     size_t build_smem = 0;
     int32_t *chain_starts = nullptr;
     int *d_err = nullptr;
@@ -297,6 +296,29 @@ void row_tiling(const gcr_ctx *c, const gcr_system_desc &d, int64_t nc, SysP &p)
     p.n_row_tiles = (int32_t)(rows * ((nc + T - 1) / T));
 }
 
+// SysP::fc from its FP64 parameters
+void set_force_consts(const gcr_ctx *c, SysP &p)
+{
+    double v[kCCount] = {};
+    v[kCRc2] = p.rc2;
+    v[kCP0] = p.p0;
+    v[kCP1] = p.p1;
+    v[kCShift] = p.shift;
+    v[kCK] = p.k;
+    v[kCKappa] = p.kappa;
+    v[kCTheta0] = p.theta0;
+    v[kCV0] = p.v0;
+    v[kCCos] = p.cos_a;
+    v[kCSin] = p.sin_a;
+    v[kCPush] = p.push_force;
+    for (int k = 0; k < kCCount; k++) {
+        if (c->cfg.precision == GCR_FP64)
+            p.fc[k] = v[k];
+        else
+            reinterpret_cast<float *>(p.fc)[k] = (float)v[k];
+    }
+}
+
 void fill_sysp(const gcr_ctx *c, const Slot &sl, int64_t nc, double skin, SysP &p)
 {
     const gcr_system_desc &d = sl.desc;
@@ -357,6 +379,7 @@ void fill_sysp(const gcr_ctx *c, const Slot &sl, int64_t nc, double skin, SysP &
     // SRK.py:364: the projection acts only when some chain has more than 2 beads
     p.rigid = (d.rigid_rod != 0.0 && sl.longest > 2) ? d.rigid_rod : 0.0;
     p.seed = d.seed;
+    set_force_consts(c, p);
 }
 
 // the coupling fields of every resident system from the context's groups,
@@ -439,6 +462,8 @@ int apply_groups(gcr_ctx *c, bool *moved)
             rows += (int64_t)p.n_cross * p.n;
         }
     }
+    for (size_t s = 0; s < c->slots.size(); s++)
+        if (c->slots[s].used) set_force_consts(c, c->hP[s]);  // the push force
     if (rows > c->x_rows) {
         GCR_CUDA(cudaStreamSynchronize(c->stream));
         if (c->xnbr) cudaFree(c->xnbr);
@@ -584,7 +609,7 @@ int enqueue_step4(gcr_ctx *c)
         void *pair = c->graph_cross ? c->ks.pair_cross[reads[k]]
                                     : (reads[k] == 0 ? c->ks.pair0 : (reads[k] == 1 ? c->ks.pair1 : c->ks.pair2));
         if ((rc = launch(c, pair, c->grid_pair, bb, c->pair_smem))) return rc;
-        if ((rc = launch(c, c->ks.stage4[k], c->grid_stage4[k], bb, c->stage_smem))) return rc;
+        if ((rc = launch(c, c->ks.stage4[k], c->grid_stage4[k], bb))) return rc;
         if (k < 3 && c->graph_rigid && (rc = launch(c, c->ks.rigid4[k], c->grid_update, bb))) return rc;
         if ((rc = launch_duty(c, k < 3 ? kDutyPlan : kDutyDt))) return rc;
     }
@@ -597,7 +622,16 @@ int enqueue_step4(gcr_ctx *c)
 // pair_mode of an SRK2 graph: 1 and 2 only without coupled populations,
 // whose cross forces only k_pair adds
 int pair_mode(const gcr_ctx *c, bool cross) { return (c->cfg.srk_order == 2 && !cross) ? c->cfg.pair_mode : 0; }
-bool fused_pair(const gcr_ctx *c, bool cross) { return pair_mode(c, cross) == 1; }
+// The stages walk the lists themselves (pair_mode 1, the same bits as 0) in 2D
+// mixed precision whatever the mode: the sweep's step takes 656 us so, 678
+// with the pair kernel.  Elsewhere only when asked for: in FP64 the 64-system
+// sweep's two stages take 233 us so, 224 with the pair kernel (registers), and
+// 3D lists are long (505 against 377 us).
+bool fused_pair(const gcr_ctx *c, bool cross)
+{
+    if (c->cfg.srk_order != 2 || cross || c->cfg.pair_mode == 2) return false;
+    return c->cfg.pair_mode == 1 || (c->cfg.dim == 2 && c->cfg.precision == GCR_MIXED);
+}
 
 // SRK2 stage s (0 predictor, 1 corrector): the pair forces, then the stage
 int enqueue_pair(gcr_ctx *c, int s, bool cross)
@@ -616,7 +650,7 @@ int enqueue_stage(gcr_ctx *c, int s, bool cross, bool rigid)
     void *stage = s == 0 ? (f ? c->ks.stage0f : c->ks.stage0) : (f ? c->ks.stage1f : c->ks.stage1);
     const int grid = s == 0 ? (f ? c->grid_stage0f : c->grid_stage0) : (f ? c->grid_stage1f : c->grid_stage1);
     const int bb = c->cfg.block_beads;
-    int rc = launch(c, stage, grid, bb, c->stage_smem);
+    int rc = launch(c, stage, grid, bb, f ? c->pair_smem : 0);
     if (!rc && s == 0 && rigid) rc = launch(c, c->ks.rigid0, c->grid_update, bb);
     return rc ? rc : launch_duty(c, s == 0 ? kDutyPlan : kDutyDt);
 }
@@ -866,21 +900,18 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     a.tile_beads = cfg.block_beads;
     a.tile_cells = cfg.block_cells;
     a.order = cfg.srk_order;
-    c->stage_smem = c->ks.stage_smem(cfg.block_beads);
-    if (c->stage_smem > 48 * 1024) {
-        cudaFuncSetAttribute(c->ks.stage0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->stage_smem);
-        cudaFuncSetAttribute(c->ks.stage1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->stage_smem);
-        cudaFuncSetAttribute(c->ks.stage0f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->stage_smem);
-        cudaFuncSetAttribute(c->ks.stage1f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->stage_smem);
-        for (int k = 0; k < 4; k++)
-            cudaFuncSetAttribute(c->ks.stage4[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->stage_smem);
-    }
+    a.mixed = cfg.precision == GCR_MIXED ? 1 : 0;
+    c->pair_smem = c->ks.pair_smem(cfg.block_beads);
+    if (c->pair_smem > 48 * 1024)
+        for (void *fn : {c->ks.pair0, c->ks.pair1, c->ks.pair2, c->ks.pair_cross[0], c->ks.pair_cross[1],
+                         c->ks.pair_cross[2], c->ks.stage0f, c->ks.stage1f})
+            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->pair_smem);
     for (int k = 0; k < 4; k++)
-        c->grid_stage4[k] = kernel_grid(c, c->ks.stage4[k], cfg.block_beads, c->max_bead_tiles, c->stage_smem);
-    c->grid_stage0 = kernel_grid(c, c->ks.stage0, cfg.block_beads, c->max_bead_tiles, c->stage_smem);
-    c->grid_stage1 = kernel_grid(c, c->ks.stage1, cfg.block_beads, c->max_bead_tiles, c->stage_smem);
-    c->grid_stage0f = kernel_grid(c, c->ks.stage0f, cfg.block_beads, c->max_bead_tiles, c->stage_smem);
-    c->grid_stage1f = kernel_grid(c, c->ks.stage1f, cfg.block_beads, c->max_bead_tiles, c->stage_smem);
+        c->grid_stage4[k] = kernel_grid(c, c->ks.stage4[k], cfg.block_beads, c->max_bead_tiles);
+    c->grid_stage0 = kernel_grid(c, c->ks.stage0, cfg.block_beads, c->max_bead_tiles);
+    c->grid_stage1 = kernel_grid(c, c->ks.stage1, cfg.block_beads, c->max_bead_tiles);
+    c->grid_stage0f = kernel_grid(c, c->ks.stage0f, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
+    c->grid_stage1f = kernel_grid(c, c->ks.stage1f, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
     c->pair_cells_smem = c->ks.pair_cells_smem(a.cell_stage_cap);
     if (c->pair_cells_smem > 48 * 1024)
         for (int k = 0; k < 2; k++)
@@ -892,7 +923,6 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
                                          2 * cfg.bead_capacity / cfg.block_beads + S,
                                      c->pair_cells_smem);
     c->grid_update = kernel_grid(c, c->ks.update, cfg.block_beads, c->max_bead_tiles);
-    c->pair_smem = c->ks.pair_smem(cfg.block_beads);
     c->grid_pair = kernel_grid(c, c->ks.pair0, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
     c->grid_bin = kernel_grid(c, c->ks.bin0, cfg.block_beads, c->max_bead_tiles);
     c->grid_sort = kernel_grid(c, c->ks.sort, cfg.block_cells, c->max_cell_tiles);

@@ -109,7 +109,14 @@ struct SysP {
     int32_t pushed;      // 1: chains pushed by a motor population
     double mparams[5];   // motors: [motor_max_dist_sq, b_one_motor_per_bead, imparts_force, k_on, k_off]
     double push_force;   // chains: the pushing motors' imparts_force
+    // the force constants in the context's force type (float, or double):
+    // read as they are, where a conversion in each thread would go through
+    // the slow conversion pipe.  Indices kC...
+    alignas(16) double fc[12];
 };
+
+// SysP::fc, entries of the force type
+enum { kCRc2, kCP0, kCP1, kCShift, kCK, kCKappa, kCTheta0, kCV0, kCCos, kCSin, kCPush, kCCount };
 
 struct SysS {
     double dt;          // predictor dt of the coming step (status.dt)
@@ -135,7 +142,39 @@ struct SysS {
     int64_t series_cap;
     int64_t series_rows;
     int64_t series_mark;  // steps_done of the last row
+    // the step's coefficients in the force type (kS...), set once per system
+    // and step instead of a division and a square root in each thread
+    alignas(16) double sc[6];
 };
+
+// SysS::sc, entries of the force type: dt / r and sqrt(2 D dt) of the
+// predictor; dt_used pref / r, sqrt(2 D dt_used) and pi sqrt(2 Dr dt_used)
+// of the update
+enum { kSPred, kSPredNoise, kSUpd, kSUpdNoise, kSUpdRot };
+
+template <typename FT>
+__host__ __device__ __forceinline__ const FT *force_consts(const SysP &p)
+{
+    return reinterpret_cast<const FT *>(p.fc);
+}
+template <typename FT>
+__device__ __forceinline__ const FT *step_consts(const SysS &s)
+{
+    return reinterpret_cast<const FT *>(s.sc);
+}
+__device__ __forceinline__ void set_step_const(SysS &s, bool mixed, int k, double v)
+{
+    if (mixed)
+        reinterpret_cast<float *>(s.sc)[k] = (float)v;
+    else
+        s.sc[k] = v;
+}
+// the predictor's coefficients, of the dt the coming step starts with
+__device__ __forceinline__ void set_predictor(const SysP &p, SysS &s, bool mixed)
+{
+    set_step_const(s, mixed, kSPred, s.dt / p.radius);
+    set_step_const(s, mixed, kSPredNoise, sqrt(2.0 * s.dt * p.D));
+}
 
 struct Tile {
     int32_t sys;
@@ -298,6 +337,14 @@ __device__ __forceinline__ double inbounds(double a, double b, double half_L, do
     else if (o >= half_L)
         o -= L;
     return o;
+}
+
+// minimum image of a - b, all axes
+template <int D>
+__device__ __forceinline__ void min_image(const double *a, const double *b, double half_L, double L, double *o)
+{
+#pragma unroll
+    for (int i = 0; i < D; i++) o[i] = inbounds(a[i], b[i], half_L, L);
 }
 
 // periodic images crossed by one coordinate in a real update: a bead moves

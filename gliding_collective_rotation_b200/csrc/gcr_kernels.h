@@ -35,6 +35,7 @@ struct BatchArgs {
     int tile_beads;
     int tile_cells;
     int order;     // SRK order of the context: 2 or 4
+    int mixed;     // the force type is float
     // cross lists of coupled populations: slot k of row r at xnbr[k * xstride + r]
     // (row r = x_off + c * n + bead for cross partner c), xcount[r] partners
     int *xnbr;
@@ -96,8 +97,7 @@ struct KernelSet {
     size_t (*pair_cells_smem)(int cap);  // their dynamic shared memory for `cap` staged beads
     int pair_cells_rows;  // cell rows a row tile stages (3 in 2D, 9 in 3D)
     int max_row_cells;    // cells of a row tile, at most
-    size_t (*stage_smem)(int block_beads);  // dynamic shared memory of the stage kernels
-    size_t (*pair_smem)(int block_beads);   // dynamic shared memory of the pair kernels
+    size_t (*pair_smem)(int block_beads);  // dynamic shared memory of the kernels that walk lists warp-wide
 };
 
 KernelSet kernel_set(int dim, int precision);

@@ -43,9 +43,11 @@
 namespace gcr {
 
 // ------------------------------------------------------------------------
-// bonded forces (forces.py:285-403).  A tile of TB beads stages the
-// positions of beads begin-2 .. begin+TB+1 in shared memory, computes every
-// bond (j, j+1) once and every bend once, then each bead gathers
+// bonded forces (forces.py:285-403).  A warp holds 32 beads, one a lane; a
+// lane computes the bond (b, b+1) and the bend of its bead, and takes its
+// neighbours' by shuffles.  Lanes 0 to 2 also compute the bonds b0-2, b0-1
+// and b0+32 and the bends of b0-1 and b0+32 beside the warp's beads.  Each
+// bead then gathers
 //   F -= s_{b-1} d_{b-1}; F -= bwd_{b-1}; F += s_b d_b; F += fwd_b + bwd_b;
 //   F -= fwd_{b+1}
 // which is the order in which the reference's sequential loop adds them.
@@ -69,44 +71,6 @@ struct Bonded {
 #define GCR_PAIR_CHUNK 2
 #endif
 constexpr int kPairChunk = GCR_PAIR_CHUNK;
-
-template <int D, typename FT>
-struct StageSmem {
-    using BT = typename Bonded<FT>::type;
-    double *x;     // [TB+4][D] positions, index k <-> bead begin-2+k
-    uint8_t *tp;   // [TB+4]    topology bits
-    BT *bd;        // [TB+3][D] bond vector d_j = min_image(x_j - x_{j+1}), k <-> bond begin-2+k
-    BT *bt;        // [TB+3][D] unit tangent of the bond (d itself when |d| = 0)
-    BT *bf;        // [TB+3]    spring magnitude k (a/|d| - 1), 0 when |d| = 0
-    BT *fw;        // [TB+2][D] bend "forward" term at bead begin-1+k
-    BT *bw;        // [TB+2][D] bend "backward" term
-    BT *ra;        // [TB+4]    rest length of the bead's chain
-    FT *pb;        // [TB/32][D+1][32 kPairChunk] the warps' buffers of the list walk (fused pair forces)
-    __device__ void carve(unsigned char *base, int TB)
-    {
-        x = reinterpret_cast<double *>(base);
-        bd = reinterpret_cast<BT *>(x + (size_t)(TB + 4) * D);
-        bt = bd + (size_t)(TB + 3) * D;
-        bf = bt + (size_t)(TB + 3) * D;
-        fw = bf + (TB + 3);
-        bw = fw + (size_t)(TB + 2) * D;
-        ra = bw + (size_t)(TB + 2) * D;
-        tp = reinterpret_cast<uint8_t *>(ra + (TB + 4));
-        pb = reinterpret_cast<FT *>(base + ((stage_base_bytes(TB) + 15) & ~(size_t)15));
-    }
-    static __host__ __device__ size_t stage_base_bytes(int TB)
-    {
-        return (size_t)(TB + 4) * D * sizeof(double) + (size_t)(TB + 3) * (2 * D + 1) * sizeof(BT) +
-               (size_t)(TB + 2) * 2 * D * sizeof(BT) + (size_t)(TB + 4) * sizeof(BT) + (size_t)(TB + 4);
-    }
-};
-
-template <int D, typename FT>
-size_t stage_smem_bytes(int TB)
-{
-    return ((StageSmem<D, FT>::stage_base_bytes(TB) + 15) & ~(size_t)15) +
-           (size_t)(TB / 32) * (D + 1) * 32 * kPairChunk * sizeof(FT);
-}
 
 // 1/sqrt(x): FP64 exactly as written in the reference; FP32 (mixed path) by
 // the hardware reciprocal square root (at most 2 ulp), accurate enough for
@@ -176,9 +140,9 @@ __device__ __forceinline__ bool bend(const FT *ti, const FT *tj, FT theta0, FT k
     return true;
 }
 
-// CTAs of 512 threads per SM that the bead kernels are compiled for: the 2D
-// mixed-precision kernels fit in 42 registers a thread with 3 (6 CTAs of 256
-// per SM), 64 with 2; the FP64 and 3D kernels keep the registers they need
+// CTAs of 512 threads per SM that the pair kernel is compiled for in 2D mixed
+// precision: 40 registers a thread with 3; the FP64 kernels keep the
+// registers they need
 #ifndef GCR_MIXED2D_MIN_BLOCKS
 #define GCR_MIXED2D_MIN_BLOCKS 3
 #endif
@@ -186,6 +150,18 @@ template <int D, typename FT>
 constexpr int min_blocks()
 {
     return (D == 2 && sizeof(FT) == 4) ? GCR_MIXED2D_MIN_BLOCKS : 1;
+}
+
+// Registers a thread of the stage kernels.  2D mixed: 56 (9 CTAs of 128
+// threads per SM).  With the pair walk in the stage the sweep's two stages
+// take 267 + 216 us so, 283 + 222 at 48 (spills) and about 3% more at 64.
+#ifndef GCR_STAGE2D_REGS
+#define GCR_STAGE2D_REGS 56
+#endif
+template <int D, typename FT>
+constexpr int stage_regs()
+{
+    return (D == 2 && sizeof(FT) == 4) ? GCR_STAGE2D_REGS : 128;
 }
 
 // ------------------------------------------------------------------------
@@ -274,26 +250,17 @@ __device__ __forceinline__ void cell_of(const SysP &p, const double *x, int *ci)
 template <int D>
 __device__ __forceinline__ bool left_skin_of(const SysP &p, const double *r, const double *x)
 {
-    double dd = 0.0;
+    double d[D], dd = 0.0;
+    min_image<D>(x, r, p.half_L, p.L, d);
 #pragma unroll
-    for (int i = 0; i < D; i++) {
-        double d = inbounds(x[i], r[i], p.half_L, p.L);
-        dd += d * d;
-    }
+    for (int i = 0; i < D; i++) dd += d[i] * d[i];
     return !(dd <= p.half_skin2);
 }
 
 template <int D>
 __device__ __forceinline__ bool left_skin(const SysP &p, const BatchArgs &A, int b, const double *x)
 {
-    const double *r = A.xref + (size_t)(p.bead_off + b) * D;
-    double dd = 0.0;
-#pragma unroll
-    for (int i = 0; i < D; i++) {
-        double d = inbounds(x[i], r[i], p.half_L, p.L);
-        dd += d * d;
-    }
-    return !(dd <= p.half_skin2);
+    return left_skin_of<D>(p, A.xref + (size_t)(p.bead_off + b) * D, x);
 }
 
 // the tiles a CTA works on: first, first + step, ...
@@ -494,6 +461,10 @@ __device__ __forceinline__ void sys_dt(const BatchArgs &A, int i)
     s.dt_next = dt;
     s.dt_used = dt_used;
     s.mfs = S;
+    // force_prefactor 0.5 of the SRK2 corrector; 1 for SRK4's weighted sum
+    set_step_const(s, A.mixed, kSUpd, dt_used * pref / p.radius);
+    set_step_const(s, A.mixed, kSUpdNoise, sqrt(2.0 * dt_used * p.D));
+    set_step_const(s, A.mixed, kSUpdRot, sqrt(2.0 * dt_used * p.Dr) * 3.141592653589793);
 }
 
 // per-system step bookkeeping after the corrector (SRK.py:330, 348-349,
@@ -503,6 +474,7 @@ __device__ __forceinline__ void sys_end(const BatchArgs &A, int i)
     SysS &s = A.S[i];
     if (!s.active || (s.flags & kFlagFatal)) return;
     s.dt = s.dt_next;
+    set_predictor(A.P[i], s, A.mixed);
     s.elapsed += s.dt_used;
     s.step += 1;
     s.steps_done += 1;
@@ -950,9 +922,11 @@ __device__ __forceinline__ bool pair_coeff(const SysP &p, const double *xj, cons
                                            FT shift, FT *sep, FT &coeff)
 {
     FT ds = FT(0);
+    double o[D];
+    min_image<D>(xj, xb, p.half_L, p.L, o);
 #pragma unroll
     for (int i = 0; i < D; i++) {
-        sep[i] = (FT)inbounds(xj[i], xb[i], p.half_L, p.L);
+        sep[i] = (FT)o[i];
         ds += sep[i] * sep[i];
     }
     const bool in = FT(0) < ds && ds <= rc2;
@@ -1010,6 +984,15 @@ __device__ __forceinline__ void pair_term(const SysP &p, const double *xj, const
 #define GCR_PAIR3D_MIN_BLOCKS 2
 #endif
 constexpr int kRowBusy = GCR_PAIR_ROW_BUSY;
+// Partners in flight in a walked row.  3D lists are long and their gathers
+// miss: four take the pair kernel of a million LJ beads from 155 to 135 us.
+// In 2D mixed precision they cost registers and gain nothing (500k LJ beads 79
+// against 80 us).
+template <int D>
+constexpr int row_ahead()
+{
+    return D == 3 ? 4 : 1;
+}
 
 template <int D, typename FT>
 size_t pair_smem_bytes(int TB)
@@ -1022,12 +1005,13 @@ __device__ __forceinline__ void warp_list_pair_force(const BatchArgs &A, const S
                                                      const double *xb, int b, int cnt, FT *F, bool &bad, FT *buf)
 {
     constexpr unsigned kAll = 0xffffffffu;
-    constexpr int C = kPairChunk, Q = 32 * C;
+    constexpr int C = kPairChunk, Q = 32 * C, U = row_ahead<D>();
     const int lane = threadIdx.x & 31;
     cnt = cnt < 0 ? 0 : (cnt < A.list_depth ? cnt : A.list_depth);
     const int n = p.n;
     const int64_t stride = A.list_stride;
-    const FT rc2 = (FT)p.rc2, p0 = (FT)p.p0, p1 = (FT)p.p1, shift = (FT)p.shift;
+    const FT *fc = force_consts<FT>(p);
+    const FT rc2 = fc[kCRc2], p0 = fc[kCP0], p1 = fc[kCP1], shift = fc[kCShift];
     // the busy rows, walked bead by bead
     int rows = 0;
     if (__reduce_add_sync(kAll, (unsigned)cnt) > (unsigned)Q)
@@ -1035,15 +1019,36 @@ __device__ __forceinline__ void warp_list_pair_force(const BatchArgs &A, const S
     {
         const int m = cnt < rows ? cnt : rows;
         const int *nb = A.nbr + p.bead_off + b;
-        int j_next = m > 0 ? nb[0] : 0;
-        for (int k = 0; k < m; k++) {
-            const int j = j_next;
-            if (k + 1 < m) j_next = nb[(size_t)(k + 1) * stride];
-            if ((unsigned)j >= (unsigned)n) {
-                bad = true;
-                continue;
+        if constexpr (U == 1) {
+            int j_next = m > 0 ? nb[0] : 0;
+            for (int k = 0; k < m; k++) {
+                const int j = j_next;
+                if (k + 1 < m) j_next = nb[(size_t)(k + 1) * stride];
+                if ((unsigned)j >= (unsigned)n) {
+                    bad = true;
+                    continue;
+                }
+                pair_term<D, FT>(p, X + (size_t)j * D, xb, rc2, p0, p1, shift, F);
             }
-            pair_term<D, FT>(p, X + (size_t)j * D, xb, rc2, p0, p1, shift, F);
+        } else {
+            for (int k = 0; k < m; k += U) {
+                int j[U];
+                double xj[U][D];
+#pragma unroll
+                for (int u = 0; u < U; u++) j[u] = k + u < m ? nb[(size_t)(k + u) * stride] : -1;
+#pragma unroll
+                for (int u = 0; u < U; u++)
+#pragma unroll
+                    for (int i = 0; i < D; i++)
+                        xj[u][i] = (unsigned)j[u] < (unsigned)n ? X[(size_t)j[u] * D + i] : 0.0;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if ((unsigned)j[u] < (unsigned)n)
+                        pair_term<D, FT>(p, xj[u], xb, rc2, p0, p1, shift, F);
+                    else
+                        bad |= k + u < m;
+                }
+            }
         }
     }
     // the tails, flattened
@@ -1416,14 +1421,14 @@ __device__ __forceinline__ void noise_rot(const SysP &p, const SysS &s, int b, F
 // pos + dt_eff F + s2 xi, wrapped; FP64 in the reference's operation order,
 // mixed: the increment in FP32 and the accumulation in FP64
 template <typename FT>
-__device__ __forceinline__ double srk_update(double x, double dt_eff, double s2, FT f, FT xi, double L)
+__device__ __forceinline__ double srk_update(double x, FT dt_eff, FT s2, FT f, FT xi, double L)
 {
     double tmp;
     if constexpr (sizeof(FT) == 8) {
         tmp = x + dt_eff * f;
         if (s2 != 0.0) tmp += s2 * xi;
     } else {
-        float inc = (float)dt_eff * f + (float)s2 * xi;
+        float inc = dt_eff * f + s2 * xi;
         tmp = x + (double)inc;
     }
     return py_mod(tmp, L);
@@ -1434,247 +1439,264 @@ __device__ __forceinline__ double srk_update(double x, double dt_eff, double s2,
 // lists itself (warp_list_pair_force, the same sums as k_pair) instead of
 // reading fp, which saves the pair kernel's launch, its second read of the
 // positions and the fp round trip (SRK2 without coupled populations only;
-// gcr_config.pair_mode 1).
+// gcr_config.pair_mode 1, and 2D mixed precision).
+// Bound by issue and by the latency of dependent loads.  A warp works on its
+// own: with the bonds and bends staged in shared memory, four CTA barriers a
+// tile and a division, a square root and a dozen conversions of constants in
+// every thread, pair and stage took 98 + 188 and 98 + 133 us on the 256-system
+// sweep; so 267 and 216 us (B200, 2D mixed, the pair walk in the stage).
+// Fetching the partners' ids and positions while the noise and the bonded terms
+// are computed cost more in registers than it hid (267 -> 370 us).
 // ------------------------------------------------------------------------
+// products that no contraction may take into a sum
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// a bond's vector d = x0 - x1, unit tangent (d itself when |d| = 0) and
+// spring magnitude k (a / |d| - 1), zeros where there is no bond
+template <int D, typename BT>
+__device__ __forceinline__ void bond(const SysP &p, bool has, const double *x0, const double *x1, BT a, BT kspring,
+                                     BT *d, BT *tt, BT &f)
+{
+    f = BT(0);
+#pragma unroll
+    for (int i = 0; i < D; i++) d[i] = tt[i] = BT(0);
+    if (!has) return;
+    double o[D];
+    min_image<D>(x0, x1, p.half_L, p.L, o);
+    BT r2 = BT(0);
+#pragma unroll
+    for (int i = 0; i < D; i++) {
+        d[i] = (BT)o[i];
+        r2 += d[i] * d[i];
+    }
+    if (r2 != BT(0)) {
+        BT inv = inv_sqrt<BT>(r2);
+        f = kspring * (a * inv - BT(1));
+#pragma unroll
+        for (int i = 0; i < D; i++) tt[i] = d[i] * inv;
+    } else {
+#pragma unroll
+        for (int i = 0; i < D; i++) tt[i] = d[i];
+    }
+}
+
 template <int D, typename FT, int STAGE, bool FUSED>
 __device__ __forceinline__ void stage_tiles(const BatchArgs &A, Span sp)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ unsigned long long sh_bits[16];
-    __shared__ int sh_run;
-    const int TB = blockDim.x;
-    StageSmem<D, FT> sm;
-    using BT = typename StageSmem<D, FT>::BT;
-    sm.carve(smem_raw, TB);
+    using BT = typename Bonded<FT>::type;
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr uint8_t kInner = kHasPrev | kHasNext;
+    const int lane = threadIdx.x & 31;
     const int nt = *A.n_bead_tiles;
     // the next tile's table entry is loaded while the current tile runs
     Tile nx = sp.first < nt ? A.bead_tiles[sp.first] : Tile{0, 0};
     for (int t = sp.first; t < nt; t += sp.step) {
-        __syncthreads();  // the previous tile is done with shared memory
         const Tile tl = nx;
         if (t + sp.step < nt) nx = A.bead_tiles[t + sp.step];
         const SysP &p = A.P[tl.sys];
         SysS &s = A.S[tl.sys];
-        // the system's constants are read before the barrier, with its flags
         const int n = p.n;
-        const int base = tl.begin - 2;
+        const int b = tl.begin + (int)threadIdx.x, b0 = b - lane;
+        if (b0 >= n) continue;  // the whole warp is past the system
+        const bool ok = b < n;
+        const int bc = ok ? b : n - 1;
         const double *X = stage_x<stage_reads(STAGE)>(p);
-        // one decision per CTA: other CTAs may raise the system's flags while
-        // this one runs, and every thread must reach the same barriers
-        if (threadIdx.x == 0) sh_run = ld_volatile(&s.active) && !(ld_volatile(&s.flags) & kFlagFatal);
-        __syncthreads();
-        if (!sh_run) continue;
-        // 1. positions and topology of beads begin-2 .. begin+TB+1
-        for (int k = threadIdx.x; k < TB + 4; k += TB) {
-            int m = base + k;
-            if (m >= 0 && m < n) {
-#pragma unroll
-                for (int i = 0; i < D; i++) sm.x[k * D + i] = X[(size_t)m * D + i];
-                sm.tp[k] = A.topo[p.bead_off + m];
-                sm.ra[k] = p.calc_springs ? (BT)A.restb[p.bead_off + m] : BT(0);
-            } else {
-                sm.tp[k] = 0;
-                sm.ra[k] = BT(0);
-            }
-        }
-        __syncthreads();
-        // the bead's own inputs of phase 4, loaded before the barriers (the
-        // build positions of a virtual update's skin test too: loaded after
-        // the pos1 stores, they would wait behind them)
-        FT pre_t[D], pre_f[D], pre_p[D];
-        double pre_r[D];
-        int pre_cnt = 0;  // list count of the fused pair walk
-        {
-            const int bq = tl.begin + (int)threadIdx.x;
-            const bool ok = bq < n;
-            const FT *tq = reinterpret_cast<const FT *>(p.tan);
-            const FT *fq = reinterpret_cast<const FT *>(p.frc);
-            const FT *pq = reinterpret_cast<const FT *>(A.fp) + (size_t)(p.bead_off + (ok ? bq : 0)) * D;
-#pragma unroll
-            for (int i = 0; i < D; i++) {
-                pre_t[i] = ok ? tq[(size_t)bq * D + i] : FT(0);
-                pre_f[i] = (ok && STAGE == 1) ? fq[(size_t)bq * D + i] : FT(0);
-                pre_p[i] = (!FUSED && ok && p.calc_wca) ? pq[i] : FT(0);
-            }
-            if constexpr (stage_writes(STAGE) != 0) {
-                const double *rq = A.xref + (size_t)(p.bead_off + (ok ? bq : 0)) * D;
-#pragma unroll
-                for (int i = 0; i < D; i++) pre_r[i] = (ok && p.calc_wca) ? rq[i] : 0.0;
-            }
-            if constexpr (FUSED) pre_cnt = (ok && p.calc_wca && !p.motor) ? A.ncount[p.bead_off + bq] : 0;
-        }
         const bool springs = p.calc_springs, cb = p.calc_bend;
+        // One decision per warp (its lanes shuffle): other warps may raise
+        // the system's flags while this one runs.  Every input is loaded
+        // before the first use: no barrier holds them apart.
+        const bool run = ld_volatile(&s.active) && !(ld_volatile(&s.flags) & kFlagFatal);
+        // 1. inputs of the lane's bead and bond, and of the bonds beside the
+        // warp (lanes 0-2: bonds b0-2, b0-1, b0+32)
+        const int64_t g = p.bead_off + bc;
+        double xb[3] = {0.0, 0.0, 0.0}, xn[D], hx[D], hn[D];
+        uint8_t tp = 0, htp = 0;
+        BT ra = BT(0), hra = BT(0);
+#pragma unroll
+        for (int i = 0; i < D; i++) {
+            xb[i] = X[(size_t)bc * D + i];
+            xn[i] = hx[i] = hn[i] = 0.0;
+        }
         if (springs) {
-            // 2. every bond (j, j+1) of the tile once
-            const BT kspring = (BT)p.k;
-            for (int k = threadIdx.x; k < TB + 3; k += TB) {
-                BT d[D], tt[D], f = BT(0);
+            const int b1 = b + 1 < n ? b + 1 : n - 1;
+            const int hb = lane < 2 ? b0 - 2 + lane : b0 + 32;
+            tp = ok ? A.topo[g] : 0;
+            ra = (BT)A.restb[g];
 #pragma unroll
-                for (int i = 0; i < D; i++) d[i] = tt[i] = BT(0);
-                if (sm.tp[k] & kHasNext) {
-                    BT r2 = BT(0);
-#pragma unroll
-                    for (int i = 0; i < D; i++) {
-                        d[i] = (BT)inbounds(sm.x[k * D + i], sm.x[(k + 1) * D + i], p.half_L, p.L);
-                        r2 += d[i] * d[i];
-                    }
-                    if (r2 != BT(0)) {
-                        const BT a = sm.ra[k];
-                        BT inv = inv_sqrt<BT>(r2);
-                        f = kspring * (a * inv - BT(1));
-#pragma unroll
-                        for (int i = 0; i < D; i++) tt[i] = d[i] * inv;
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < D; i++) tt[i] = d[i];
-                    }
-                }
+            for (int i = 0; i < D; i++) xn[i] = X[(size_t)b1 * D + i];
+            if (lane < 3 && hb >= 0 && hb < n) {
+                htp = A.topo[p.bead_off + hb];
+                hra = (BT)A.restb[p.bead_off + hb];
+                const int h1 = hb + 1 < n ? hb + 1 : n - 1;
 #pragma unroll
                 for (int i = 0; i < D; i++) {
-                    sm.bd[k * D + i] = d[i];
-                    sm.bt[k * D + i] = tt[i];
-                }
-                sm.bf[k] = f;
-            }
-            __syncthreads();
-            // 3. every bend once: bead begin-1+k uses bonds k+1 (own) and k
-            if (cb) {
-                const BT kappa = (BT)p.kappa, theta0 = (BT)p.theta0;
-                for (int k = threadIdx.x; k < TB + 2; k += TB) {
-                    BT fw[D], bw[D];
-#pragma unroll
-                    for (int i = 0; i < D; i++) fw[i] = bw[i] = BT(0);
-                    const uint8_t tp = sm.tp[k + 1];
-                    if ((tp & kHasPrev) && (tp & kHasNext)) {
-                        if (!bend<D, BT>(sm.bt + (k + 1) * D, sm.bt + k * D, theta0, kappa, fw, bw)) {
-#pragma unroll
-                            for (int i = 0; i < D; i++) fw[i] = bw[i] = BT(0);
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < D; i++) {
-                        sm.fw[k * D + i] = fw[i];
-                        sm.bw[k * D + i] = bw[i];
-                    }
+                    hx[i] = X[(size_t)hb * D + i];
+                    hn[i] = X[(size_t)h1 * D + i];
                 }
             }
-            __syncthreads();
         }
-        // 4. per bead: gather bonded terms, pair forces, propulsion, update
-        const int tid = threadIdx.x;
-        const int b = tl.begin + tid;
-        // fused pair forces: the warp-wide list walk of k_pair, which every
-        // lane of the warp joins (a lane past the system with no list)
+        FT *frc = reinterpret_cast<FT *>(p.frc);
+        FT *tan = reinterpret_cast<FT *>(p.tan);
+        FT tg[3] = {FT(0), FT(0), FT(0)};
+        BT Fb[3] = {BT(0), BT(0), BT(0)};
         FT Fp[3] = {FT(0), FT(0), FT(0)};
-        if constexpr (FUSED) {
-            if (p.calc_wca) {
-                bool bad = false;
-                double xq[3] = {0.0, 0.0, 0.0};
+        double pre_r[D];  // build position, for the skin test of a virtual update
+        int cnt = 0;      // list count of the fused pair walk
 #pragma unroll
-                for (int i = 0; i < D; i++) xq[i] = sm.x[(tid + 2) * D + i];
-                warp_list_pair_force<D, FT>(A, p, X, xq, b, pre_cnt, Fp, bad,
-                                            sm.pb + (size_t)(tid >> 5) * (D + 1) * 32 * kPairChunk);
-                if (bad) atomicOr(&s.flags, kFlagListCorrupt);
-            }
+        for (int i = 0; i < D; i++) {
+            // a bead of a chain takes its tangent from its bonds below
+            if (!p.get_orient) tg[i] = tan[(size_t)bc * D + i];
+            // the SRK2 corrector adds to F0; every other stage starts from 0
+            if (STAGE == 1) Fb[i] = (BT)frc[(size_t)bc * D + i];
+            if (!FUSED && p.calc_wca) Fp[i] = reinterpret_cast<const FT *>(A.fp)[(size_t)g * D + i];
+            pre_r[i] = stage_writes(STAGE) != 0 && p.calc_wca ? A.xref[(size_t)g * D + i] : 0.0;
         }
-        double mf2 = 0.0;
-        if (b < n) {
-            FT *frc = reinterpret_cast<FT *>(p.frc);
-            FT *tan = reinterpret_cast<FT *>(p.tan);
-            double xb[3] = {0.0, 0.0, 0.0};
+        if constexpr (FUSED) cnt = (ok && p.calc_wca && !p.motor) ? A.ncount[g] : 0;
+        if (!__shfl_sync(kAll, run, 0)) continue;
+        const FT *fc = force_consts<FT>(p);
+        bool tang_set = false;
+        if (springs) {
+            // 2. bonds
+            const BT kspring = sizeof(BT) == sizeof(FT) ? (BT)fc[kCK] : (BT)p.k;
+            BT d[D], tt[D], f, hd[D], ht[D], hf = BT(0);
+            bond<D, BT>(p, tp & kHasNext, xb, xn, ra, kspring, d, tt, f);
 #pragma unroll
-            for (int i = 0; i < D; i++) xb[i] = sm.x[(tid + 2) * D + i];
-            // F0 (stage 1) and the bonded terms summed in BT, then FT
-            BT Fb[3];
-            FT F[3], tg[3];
+            for (int i = 0; i < D; i++) hd[i] = ht[i] = BT(0);
+            if (lane < 3) bond<D, BT>(p, htp & kHasNext, hx, hn, hra, kspring, hd, ht, hf);
+            __syncwarp();
+            // the bond before the lane's
+            BT dm[D], tj[D], fm;
 #pragma unroll
             for (int i = 0; i < D; i++) {
-                // the SRK2 corrector adds to F0; every other stage starts from 0
-                Fb[i] = STAGE == 1 ? (BT)pre_f[i] : BT(0);
-                tg[i] = pre_t[i];
+                const BT du = __shfl_up_sync(kAll, d[i], 1), dh = __shfl_sync(kAll, hd[i], 1);
+                const BT tu = __shfl_up_sync(kAll, tt[i], 1), th = __shfl_sync(kAll, ht[i], 1);
+                dm[i] = lane == 0 ? dh : du;
+                tj[i] = lane == 0 ? th : tu;
             }
-            bool tang_set = false;
-            if (springs) {
-                const uint8_t tp = sm.tp[tid + 2];
-                const bool prev = tp & kHasPrev, next = tp & kHasNext;
-                if (prev) {
-                    const BT f = sm.bf[tid + 1];
+            {
+                const BT fu = __shfl_up_sync(kAll, f, 1), fh = __shfl_sync(kAll, hf, 1);
+                fm = lane == 0 ? fh : fu;
+            }
+            // 3. bends: of the lane's bead, and of b0-1 (lane 1) and b0+32 (lane 2)
+            BT fw[D], bw[D], bwm[D], fwp[D];
 #pragma unroll
-                    for (int i = 0; i < D; i++) Fb[i] -= sm.bd[(tid + 1) * D + i] * f;
-                    if ((tp & kHasPrev2) && cb) {
+            for (int i = 0; i < D; i++) fw[i] = bw[i] = bwm[i] = fwp[i] = BT(0);
+            if (cb) {
+                const BT kappa = sizeof(BT) == sizeof(FT) ? (BT)fc[kCKappa] : (BT)p.kappa;
+                const BT theta0 = sizeof(BT) == sizeof(FT) ? (BT)fc[kCTheta0] : (BT)p.theta0;
+                if ((tp & kInner) == kInner && !bend<D, BT>(tt, tj, theta0, kappa, fw, bw)) {
 #pragma unroll
-                        for (int i = 0; i < D; i++) Fb[i] -= sm.bw[tid * D + i];
-                    }
+                    for (int i = 0; i < D; i++) fw[i] = bw[i] = BT(0);
                 }
-                if (next) {
-                    const BT f = sm.bf[tid + 2];
+                __syncwarp();
+                BT hj[D], hfw[D], hbw[D];
 #pragma unroll
-                    for (int i = 0; i < D; i++) Fb[i] += sm.bd[(tid + 2) * D + i] * f;
+                for (int i = 0; i < D; i++) {
+                    const BT t0 = __shfl_sync(kAll, ht[i], 0), t31 = __shfl_sync(kAll, tt[i], 31);
+                    hj[i] = lane == 1 ? t0 : t31;
+                    hfw[i] = hbw[i] = BT(0);
                 }
-                if (prev && next && cb) {
+                if ((lane == 1 || lane == 2) && (htp & kInner) == kInner &&
+                    !bend<D, BT>(ht, hj, theta0, kappa, hfw, hbw)) {
 #pragma unroll
-                    for (int i = 0; i < D; i++) Fb[i] += sm.fw[(tid + 1) * D + i] + sm.bw[(tid + 1) * D + i];
+                    for (int i = 0; i < D; i++) hfw[i] = hbw[i] = BT(0);
                 }
-                if ((tp & kHasNext2) && cb) {
+                __syncwarp();
 #pragma unroll
-                    for (int i = 0; i < D; i++) Fb[i] -= sm.fw[(tid + 2) * D + i];
-                }
-                if (p.get_orient && (prev || next)) {
-                    const BT *ti = sm.bt + (tid + 2) * D, *tj = sm.bt + (tid + 1) * D;
-                    if (prev && next) {
-                        // (ti + tj) / sqrt(2 (1 + c)); aligned tangents give ti.  In
-                        // FP32 1 + c = 2 - |tj - ti|^2 / 2 and the aligned test
-                        // from the chord, as in bend()
-                        bool interior;
-                        BT coeff;
-                        if constexpr (sizeof(BT) == 4) {
-                            BT ch2 = BT(0);
-#pragma unroll
-                            for (int i = 0; i < D; i++) ch2 += (tj[i] - ti[i]) * (tj[i] - ti[i]);
-                            const BT omc = BT(0.5) * ch2;
-                            interior = omc > BT(0) && omc < BT(2);
-                            coeff = inv_sqrt<BT>(BT(2) * (BT(2) - omc));
-                        } else {
-                            BT c = BT(0);
-#pragma unroll
-                            for (int i = 0; i < D; i++) c += ti[i] * tj[i];
-                            interior = BT(-1) < c && c < BT(1);
-                            coeff = inv_sqrt<BT>(BT(2) * (BT(1) + c));
-                        }
-                        if (interior) {
-#pragma unroll
-                            for (int i = 0; i < D; i++) tg[i] = (FT)(coeff * (ti[i] + tj[i]));
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < D; i++) tg[i] = (FT)ti[i];
-                        }
-                    } else if (next) {  // head bead
-#pragma unroll
-                        for (int i = 0; i < D; i++) tg[i] = (FT)ti[i];
-                    } else {  // tail bead
-#pragma unroll
-                        for (int i = 0; i < D; i++) tg[i] = (FT)tj[i];
-                    }
-                    tang_set = true;
+                for (int i = 0; i < D; i++) {
+                    const BT u = __shfl_up_sync(kAll, bw[i], 1), uh = __shfl_sync(kAll, hbw[i], 1);
+                    const BT w = __shfl_down_sync(kAll, fw[i], 1), wh = __shfl_sync(kAll, hfw[i], 2);
+                    bwm[i] = lane == 0 ? uh : u;
+                    fwp[i] = lane == 31 ? wh : w;
                 }
             }
+            // 4. the bonded terms of the bead
+            const bool prev = tp & kHasPrev, next = tp & kHasNext;
+            if (prev) {
+#pragma unroll
+                for (int i = 0; i < D; i++) Fb[i] -= dm[i] * fm;
+                if ((tp & kHasPrev2) && cb) {
+#pragma unroll
+                    for (int i = 0; i < D; i++) Fb[i] -= bwm[i];
+                }
+            }
+            if (next) {
+#pragma unroll
+                for (int i = 0; i < D; i++) Fb[i] += d[i] * f;
+            }
+            if (prev && next && cb) {
+#pragma unroll
+                for (int i = 0; i < D; i++) Fb[i] += fw[i] + bw[i];
+            }
+            if ((tp & kHasNext2) && cb) {
+#pragma unroll
+                for (int i = 0; i < D; i++) Fb[i] -= fwp[i];
+            }
+            if (p.get_orient) {
+                if (prev && next) {
+                    // (ti + tj) / sqrt(2 (1 + c)); aligned tangents give ti.  In
+                    // FP32 1 + c = 2 - |tj - ti|^2 / 2 and the aligned test
+                    // from the chord, as in bend()
+                    bool interior;
+                    BT coeff;
+                    if constexpr (sizeof(BT) == 4) {
+                        BT ch2 = BT(0);
+#pragma unroll
+                        for (int i = 0; i < D; i++) ch2 += (tj[i] - tt[i]) * (tj[i] - tt[i]);
+                        const BT omc = BT(0.5) * ch2;
+                        interior = omc > BT(0) && omc < BT(2);
+                        coeff = inv_sqrt<BT>(BT(2) * (BT(2) - omc));
+                    } else {
+                        BT c = BT(0);
+#pragma unroll
+                        for (int i = 0; i < D; i++) c += tt[i] * tj[i];
+                        interior = BT(-1) < c && c < BT(1);
+                        coeff = inv_sqrt<BT>(BT(2) * (BT(1) + c));
+                    }
+#pragma unroll
+                    for (int i = 0; i < D; i++) tg[i] = interior ? (FT)(coeff * (tt[i] + tj[i])) : (FT)tt[i];
+                } else if (next) {  // head bead
+#pragma unroll
+                    for (int i = 0; i < D; i++) tg[i] = (FT)tt[i];
+                } else if (prev) {  // tail bead
+#pragma unroll
+                    for (int i = 0; i < D; i++) tg[i] = (FT)tj[i];
+                } else if (ok) {  // a chain of one bead keeps its tangent
+#pragma unroll
+                    for (int i = 0; i < D; i++) tg[i] = tan[(size_t)b * D + i];
+                }
+                tang_set = prev || next;
+            }
+        }
+        // 5. the fused pair forces: every lane of the warp joins (a lane past
+        // the system with no list)
+        if constexpr (FUSED) {
+            __syncwarp();
+            bool bad = false;
+            warp_list_pair_force<D, FT>(A, p, X, xb, b, cnt, Fp, bad,
+                                        reinterpret_cast<FT *>(smem_raw) +
+                                            (size_t)(threadIdx.x >> 5) * (D + 1) * 32 * kPairChunk);
+            if (bad) atomicOr(&s.flags, kFlagListCorrupt);
+        }
+        double mf2 = 0.0;
+        if (ok) {
+            FT F[3];
 #pragma unroll
             for (int i = 0; i < D; i++) F[i] = (FT)Fb[i];
             if (p.calc_wca) {
-                if constexpr (FUSED) {
 #pragma unroll
-                    for (int i = 0; i < D; i++) F[i] += Fp[i];
-                } else {
-#pragma unroll
-                    for (int i = 0; i < D; i++) F[i] += pre_p[i];
-                }
+                for (int i = 0; i < D; i++) F[i] += Fp[i];
             }
             if (p.self_propel) {
-                const FT v0 = (FT)p.v0;
+                const FT v0 = fc[kCV0];
                 if (p.rotate_prop) {
-                    const FT cs = (FT)p.cos_a, sn = (FT)p.sin_a;
-                    FT fx = v0 * (cs * tg[0] - sn * tg[1]);
-                    FT fy = v0 * (sn * tg[0] + cs * tg[1]);
+                    const FT cs = fc[kCCos], sn = fc[kCSin];
+                    // (the contraction is written out: every kernel that
+                    // holds this sum rounds it alike)
+                    FT fx = v0 * fma(cs, tg[0], -mul_rn(sn, tg[1]));
+                    FT fy = v0 * fma(cs, tg[1], mul_rn(sn, tg[0]));
                     F[0] += fx;
                     F[1] += fy;
                 } else {
@@ -1688,14 +1710,14 @@ __device__ __forceinline__ void stage_tiles(const BatchArgs &A, Span sp)
                     // the chains' own forces as the other population's
                     // force (SRK.py:261-267, 287-294); where_active counts
                     // the attached motors from -1 at each step (SRK.py:132)
-                    int *mp = A.mpush + p.bead_off + b, *md = A.mdelta + p.bead_off + b;
+                    int *mp = A.mpush + g, *md = A.mdelta + g;
                     const int npush = *mp, dl = *md;
                     *mp = 0;
                     *md = 0;
-                    int *ab = A.act + p.bead_off + b;
+                    int *ab = A.act + g;
                     *ab = (STAGE == 0 ? -1 : *ab) + dl;
                     if (npush > 0) {
-                        const FT f = (FT)p.push_force;
+                        const FT f = fc[kCPush];
                         FT M[3] = {FT(0), FT(0), FT(0)};
                         for (int k = 0; k < npush; k++) {
 #pragma unroll
@@ -1722,6 +1744,24 @@ __device__ __forceinline__ void stage_tiles(const BatchArgs &A, Span sp)
 #pragma unroll
                 for (int i = 0; i < D; i++) G[i] = F[i];
             }
+            // the step's translational noise, drawn once in the first stage
+            FT xi[3] = {FT(0), FT(0), FT(0)};
+            double xo[3] = {0.0, 0.0, 0.0};
+            if constexpr (stage_writes(STAGE) != 0) {
+                if (p.D > 0.0) {
+                    if constexpr (STAGE == 0 || STAGE == 10) noise_trans<D, FT>(p, s, b, xi);
+                    FT *xs = reinterpret_cast<FT *>(A.xi) + (size_t)g * D;
+#pragma unroll
+                    for (int i = 0; i < D; i++) {
+                        if (STAGE == 0 || STAGE == 10)
+                            xs[i] = xi[i];
+                        else
+                            xi[i] = xs[i];
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < D; i++) xo[i] = stage_reads(STAGE) == 0 ? xb[i] : p.pos[(size_t)b * D + i];
+            }
 #pragma unroll
             for (int i = 0; i < D; i++) frc[(size_t)b * D + i] = G[i];
             if (tang_set) {
@@ -1729,40 +1769,25 @@ __device__ __forceinline__ void stage_tiles(const BatchArgs &A, Span sp)
                 for (int i = 0; i < D; i++) tan[(size_t)b * D + i] = tg[i];
             }
             if constexpr (stage_writes(STAGE) != 0) {
-                // the step's translational noise, drawn once in the first stage
-                FT xi[3] = {FT(0), FT(0), FT(0)};
-                if (p.D > 0.0) {
-                    FT *xs = reinterpret_cast<FT *>(A.xi) + (size_t)(p.bead_off + b) * D;
-                    if constexpr (STAGE == 0 || STAGE == 10) {
-                        noise_trans<D, FT>(p, s, b, xi);
-#pragma unroll
-                        for (int i = 0; i < D; i++) xs[i] = xi[i];
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < D; i++) xi[i] = xs[i];
-                    }
-                }
                 // virtual update: (pos + dt_eff/r F + sqrt(2 D dt) xi) mod L
                 // from the step's old positions (with the rigid-rod
                 // projection on, k_rigid writes it)
                 if (p.rigid == 0.0) {
-                    const double dt = s.dt;
-                    const double dt_eff = dt * stage_dt_factor(STAGE) / p.radius;
-                    const double s2 = sqrt(2.0 * dt * p.D);
+                    const FT *sc = step_consts<FT>(s);
+                    const FT dt_eff = sc[kSPred] * FT(stage_dt_factor(STAGE)), s2 = sc[kSPredNoise];
                     double *W = stage_x<stage_writes(STAGE)>(p);
                     double x1[3] = {0.0, 0.0, 0.0};
                     bool finite = true;
                     // an attached motor writes no virtual position: its pos1
                     // keeps the previous value (SRK.py:389-395)
-                    const bool hold = p.motor && p.motor_hold && A.act[p.bead_off + b] >= 0;
+                    const bool hold = p.motor && p.motor_hold && A.act[g] >= 0;
 #pragma unroll
                     for (int i = 0; i < D; i++) {
                         if (hold) {
                             x1[i] = W[(size_t)b * D + i];
                             continue;
                         }
-                        const double x0 = stage_reads(STAGE) == 0 ? xb[i] : p.pos[(size_t)b * D + i];
-                        x1[i] = srk_update<FT>(x0, dt_eff, s2, F[i], xi[i], p.L);
+                        x1[i] = srk_update<FT>(xo[i], dt_eff, s2, F[i], xi[i], p.L);
                         finite &= isfinite(x1[i]);
                         W[(size_t)b * D + i] = x1[i];
                     }
@@ -1781,25 +1806,23 @@ __device__ __forceinline__ void stage_tiles(const BatchArgs &A, Span sp)
             }
         }
         if (STAGE == 1 || STAGE == 13) {
-            // warp / block max over non-negative doubles via their bit patterns
-            unsigned long long bits = (unsigned long long)__double_as_longlong(mf2);
-            for (int o = 16; o > 0; o >>= 1) {
-                unsigned long long other = __shfl_xor_sync(0xffffffffu, bits, o);
-                bits = other > bits ? other : bits;
-            }
-            if ((threadIdx.x & 31) == 0) sh_bits[threadIdx.x >> 5] = bits;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                unsigned long long mx = 0;
-                for (int w = 0; w < (TB + 31) / 32; w++) mx = sh_bits[w] > mx ? sh_bits[w] : mx;
-                if (mx) atomicMax(&s.max_f2, mx);
+            // warp max over non-negative doubles via their bit patterns, high
+            // word first
+            __syncwarp();
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(mf2);
+            const unsigned hi = (unsigned)(bits >> 32), mh = __reduce_max_sync(kAll, hi);
+            const unsigned ml = __reduce_max_sync(kAll, hi == mh ? (unsigned)bits : 0u);
+            if (lane == 0) {
+                const unsigned long long mx = (unsigned long long)mh << 32 | ml;
+                // most warps find a larger force there already
+                if (mx > *(const volatile unsigned long long *)&s.max_f2) atomicMax(&s.max_f2, mx);
             }
         }
     }
 }
 
 template <int D, typename FT, int STAGE, bool FUSED = false>
-__global__ void __launch_bounds__(512, min_blocks<D, FT>()) k_stage(const __grid_constant__ BatchArgs A)
+__global__ void __maxnreg__((stage_regs<D, FT>())) k_stage(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
     stage_tiles<D, FT, STAGE, FUSED>(A, launch_span());
@@ -1858,10 +1881,8 @@ __device__ __forceinline__ void update_tiles(const BatchArgs &A, Span sp)
         }
         // no barriers in this kernel: a per-thread decision is safe
         if (!s.active || (s.flags & kFlagFatal) || !valid) continue;
-        const double dtu = s.dt_used;
-        // force_prefactor 0.5 of the SRK2 corrector; 1 for SRK4's weighted sum
-        const double dt_eff = dtu * (A.order == 4 ? 1.0 : 0.5) / p.radius;
-        const double s2 = sqrt(2.0 * dtu * p.D);
+        const FT *sc = step_consts<FT>(s);
+        const FT dt_eff = sc[kSUpd], s2 = sc[kSUpdNoise];
         double x[3] = {0.0, 0.0, 0.0};
         bool finite = true;
         // an attached motor keeps its position (SRK.py:389-395)
@@ -1890,7 +1911,7 @@ __device__ __forceinline__ void update_tiles(const BatchArgs &A, Span sp)
             FT tb[3];
 #pragma unroll
             for (int i = 0; i < D; i++) tb[i] = tan[(size_t)b * D + i];
-            const FT sq = (FT)(sqrt(2.0 * dtu * p.Dr) * 3.141592653589793);
+            const FT sq = sc[kSUpdRot];
             FT proj = FT(0);
 #pragma unroll
             for (int i = 0; i < D; i++) proj += xr[i] * tb[i];
@@ -2092,7 +2113,7 @@ __global__ void __launch_bounds__(512) k_rigid(const __grid_constant__ BatchArgs
 // r_cut.  Coupled populations are flagged outright: their fixed members have
 // no bead tiles to test.
 template <int D>
-__global__ void __launch_bounds__(512) k_run_check(BatchArgs A)
+__global__ void __launch_bounds__(512) k_run_check(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
     const int nt = *A.n_bead_tiles;
@@ -2104,6 +2125,7 @@ __global__ void __launch_bounds__(512) k_run_check(BatchArgs A)
         if (!ld_volatile(&s.active) || (ld_volatile(&s.flags) & kFlagFatal)) continue;
         const int b = tl.begin + threadIdx.x;
         if (b >= p.n || threadIdx.x >= A.tile_beads) continue;
+        if (b == 0) set_predictor(p, s, A.mixed);
         if (p.calc_springs) {
             int ch = p.chain[b];
             ch = ch < 0 ? 0 : (ch >= p.n_chains ? p.n_chains - 1 : ch);

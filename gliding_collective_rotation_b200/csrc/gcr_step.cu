@@ -77,10 +77,6 @@ KernelSet kernel_set(int dim, int precision)
 {
     KernelSet k{};
     if (dim == 2)
-        k.stage_smem = precision == 0 ? stage_smem_bytes<2, double> : stage_smem_bytes<2, float>;
-    else
-        k.stage_smem = precision == 0 ? stage_smem_bytes<3, double> : stage_smem_bytes<3, float>;
-    if (dim == 2)
         k.pair_smem = precision == 0 ? pair_smem_bytes<2, double> : pair_smem_bytes<2, float>;
     else
         k.pair_smem = precision == 0 ? pair_smem_bytes<3, double> : pair_smem_bytes<3, float>;
