@@ -2194,30 +2194,43 @@ __device__ __forceinline__ void motor_tiles(const BatchArgs &A, Span sp)
         const double r2 = p.cross_rc2[k], dmax2 = p.mparams[0], k_on = p.mparams[3], k_off = p.mparams[4];
         const int64_t step = s.step;
         bool bad = false;
-        for (int e = 0; e < cnt; e++) {
-            const int j = A.xnbr[row + (int64_t)e * A.xstride];
-            if ((unsigned)j >= (unsigned)q.n) {
-                bad = true;
-                continue;
-            }
-            double ds = 0.0;
+        // four candidates' positions in flight; a draw only where it decides
+        // something: a free motor's candidates are mostly out of its reach
+        // (16 boxes of 1800 motors and 2000 chain beads, pair and motor kernels
+        // of a stage: 34 -> 30 us)
+        constexpr int U = 4;
+        for (int e = 0; e < cnt; e += U) {
+            int j[U];
+            double ds[U];
 #pragma unroll
-            for (int i = 0; i < D; i++) {
-                const double d = inbounds(xm[i], XQ[(size_t)j * D + i], p.half_L, p.L);
-                ds = __dadd_rn(ds, __dmul_rn(d, d));
+            for (int u = 0; u < U; u++) j[u] = e + u < cnt ? A.xnbr[row + (int64_t)(e + u) * A.xstride] : -1;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const bool ok = (unsigned)j[u] < (unsigned)q.n;
+                bad |= !ok && e + u < cnt;
+                ds[u] = 0.0;
+#pragma unroll
+                for (int i = 0; i < D; i++) {
+                    const double d = inbounds(xm[i], ok ? XQ[(size_t)j[u] * D + i] : 0.0, p.half_L, p.L);
+                    ds[u] = __dadd_rn(ds[u], __dmul_rn(d, d));
+                }
+                if (!(ok && ds[u] <= r2)) j[u] = -1;
             }
-            if (!(ds <= r2)) continue;
-            double u_off, u_on;
-            motor_uniforms(p.seed, (uint32_t)m, (uint32_t)j, step, WHICH, u_off, u_on);
-            if (am >= 0) {
-                if (u_off > k_off) continue;
-                am = -1;
-                atomicAdd(A.mdelta + q.bead_off + j, -1);
-            }
-            if (am < 0 && u_on < k_on && ds <= dmax2) {
-                atomicAdd(A.mdelta + q.bead_off + j, 1);
-                atomicAdd(A.mpush + q.bead_off + j, 1);
-                am = j;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (j[u] < 0 || (am < 0 && !(ds[u] <= dmax2))) continue;
+                double u_off, u_on;
+                motor_uniforms(p.seed, (uint32_t)m, (uint32_t)j[u], step, WHICH, u_off, u_on);
+                if (am >= 0) {
+                    if (u_off > k_off) continue;
+                    am = -1;
+                    atomicAdd(A.mdelta + q.bead_off + j[u], -1);
+                }
+                if (u_on < k_on && ds[u] <= dmax2) {
+                    atomicAdd(A.mdelta + q.bead_off + j[u], 1);
+                    atomicAdd(A.mpush + q.bead_off + j[u], 1);
+                    am = j[u];
+                }
             }
         }
         *act_m = am;
