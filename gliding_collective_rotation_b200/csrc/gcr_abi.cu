@@ -148,6 +148,8 @@ struct gcr_ctx {
     size_t pair_smem = 0;
     size_t build_smem = 0;
     int32_t *chain_starts = nullptr;
+    void *corr = nullptr;  // scratch of the pair correlations (lazy): centres, angles, histograms
+    size_t corr_bytes = 0;
     int *d_err = nullptr;
     double *d_out = nullptr;
     int64_t max_bead_tiles = 0, max_cell_tiles = 0;
@@ -940,7 +942,7 @@ int gcr_destroy(gcr_ctx *c)
     if (c->graph) cudaGraphExecDestroy(c->graph);
     void *ptrs[] = {c->dP, c->dS, c->d_bead_tiles, c->d_cell_tiles, c->d_ntiles, c->d_row_prefix, c->topo, c->cnt[0],
                     c->cnt[1], c->items, c->nbr, c->ncount, c->xref, c->work, c->xi, c->fp, c->chain_starts, c->d_err,
-                    c->d_out, c->pos2, c->faux, c->xnbr, c->xcount, c->img, c->act, c->mpush, c->mdelta, c->restb};
+                    c->d_out, c->pos2, c->faux, c->xnbr, c->xcount, c->img, c->act, c->mpush, c->mdelta, c->restb, c->corr};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -1590,7 +1592,7 @@ int gcr_chain_frames(gcr_ctx *c, int32_t slot, double *com, double *phi)
     if (!valid_slot(c, slot)) return fail(GCR_ERR_BAD_ARG, "invalid slot");
     const Slot &sl = c->slots[slot];
     GCR_CUDA(launch_chain_frames(c->cfg.dim, c->cfg.precision, c->hP[slot], c->chain_starts + sl.chain_off, com, phi,
-                                 c->stream));
+                                 0, nullptr, c->stream));
     GCR_CUDA(cudaStreamSynchronize(c->stream));
     return GCR_OK;
 }
@@ -1610,25 +1612,30 @@ int gcr_pair_correlation(gcr_ctx *c, int32_t slot, int32_t kind, double binsize,
     const int nc = p.n_chains;
     if (kind != 0 && (int64_t)nc * (nc - 1) > ((int64_t)1 << 31))
         return fail(GCR_ERR_BAD_ARG, "Cvv / Cnn are limited to about 46000 chains (fixed-point sums)");
-    double *com = nullptr, *phi = nullptr;
-    unsigned long long *hist = nullptr;
-    // analysis call, not the step: its scratch is allocated here and freed below
-    cudaError_t e = cudaMalloc(&com, sizeof(double) * 2 * (size_t)nc);
-    if (e == cudaSuccess) e = cudaMalloc(&phi, sizeof(double) * 2 * (size_t)nc);
-    if (e == cudaSuccess) e = cudaMalloc(&hist, sizeof(unsigned long long) * 2 * (size_t)n_bins);
-    if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, sizeof(unsigned long long) * 2 * (size_t)n_bins, c->stream);
+    // scratch of the context, grown on demand: an allocation and a free on each
+    // call, which wait for the device, took longer than the kernels
+    const size_t need = sizeof(double) * 4 * (size_t)nc + sizeof(unsigned long long) * 2 * (size_t)n_bins;
+    if (need > c->corr_bytes) {
+        if (c->corr) cudaFree(c->corr);
+        c->corr = nullptr;
+        c->corr_bytes = 0;
+        GCR_CUDA(cudaMalloc(&c->corr, need));
+        c->corr_bytes = need;
+    }
+    double *com = (double *)c->corr, *trig = com + 2 * (size_t)nc;
+    unsigned long long *hist = (unsigned long long *)(trig + 2 * (size_t)nc);
+    cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(unsigned long long) * 2 * (size_t)n_bins, c->stream);
     if (e == cudaSuccess)
-        e = launch_chain_frames(2, c->cfg.precision, p, c->chain_starts + c->slots[slot].chain_off, com, phi, c->stream);
+        e = launch_chain_frames(2, c->cfg.precision, p, c->chain_starts + c->slots[slot].chain_off, com, nullptr, kind,
+                                kind != 0 ? trig : nullptr, c->stream);
     if (e == cudaSuccess)
-        e = launch_pair_corr(com, phi, nc, p.L, binsize, (int)n_bins, kind, hist, hist + n_bins, c->sm_count, c->stream);
+        e = launch_pair_corr(com, trig, nc, p.L, binsize, (int)n_bins, kind, hist, hist + n_bins, c->sm_count,
+                             c->stream);
     std::vector<unsigned long long> h((size_t)(2 * n_bins));
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h.data(), hist, sizeof(unsigned long long) * 2 * (size_t)n_bins, cudaMemcpyDeviceToHost,
                             c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(com);
-    cudaFree(phi);
-    cudaFree(hist);
     if (e != cudaSuccess) return fail(GCR_ERR_CUDA, std::string("pair correlation: ") + cudaGetErrorString(e));
     // normalisation of correlation_func (analysis.py:229-237), rows with r < L/2
     double total = 0.0;

@@ -121,9 +121,10 @@ cudaError_t launch_export_list(const int *nbr, const int *ncount, int64_t stride
                                int32_t *counts, int32_t *partners, int partners_depth, unsigned long long *total,
                                cudaStream_t st);
 // gcr_observables.cu
+// com, phi, trig may be null; trig: cosine and sine of the chains' angle of 1- or 2-fold symmetry (sym)
 cudaError_t launch_chain_frames(int dim, int precision, const SysP &p, const int32_t *chain_start, double *com,
-                                double *phi, cudaStream_t st);
-cudaError_t launch_pair_corr(const double *com, const double *phi, int n_chains, double L, double binsize, int n_bins,
+                                double *phi, int sym, double *trig, cudaStream_t st);
+cudaError_t launch_pair_corr(const double *com, const double *trig, int n_chains, double L, double binsize, int n_bins,
                              int kind, unsigned long long *counts, unsigned long long *sums, int sm_count,
                              cudaStream_t st);
 // out[n][dim] = pos + L * img (unwrapped positions of one system)

@@ -240,7 +240,9 @@ __device__ void order_params_block(int dim, const FT *__restrict__ tan, const in
     double ex = 0.0, ey = 0.0, q11 = 0.0, q12 = 0.0;
     for (int c = threadIdx.x; c < n_chains; c += blockDim.x) {
         double sx = 0.0, sy = 0.0;
-        for (int b = cs[c]; b < cs[c + 1]; b++) {
+        const int b0 = cs[c], b1 = cs[c + 1];
+#pragma unroll 4
+        for (int b = b0; b < b1; b++) {
             sx += (double)tan[(size_t)b * dim];
             sy += (double)tan[(size_t)b * dim + 1];
         }

@@ -43,12 +43,12 @@ def pair_correlation(engine, slot, kind="g_of_r", binsize=0.25):
     st = engine.systems[slot]
     L = float(st.params.L)
     rows = int(np.ceil(L / 2 / binsize)) + 2
-    out = (C.c_double * (2 * rows))()
+    out = np.empty((rows, 2))
     n = C.c_int32()
     torch.cuda.current_stream(st.pos.device).synchronize()
-    check(engine.lib.gcr_pair_correlation(engine._ctx, int(slot), KINDS[kind], float(binsize), out, rows,
-                                          C.byref(n)))
-    return np.array(out[:2 * n.value]).reshape(-1, 2)
+    check(engine.lib.gcr_pair_correlation(engine._ctx, int(slot), KINDS[kind], float(binsize),
+                                          out.ctypes.data_as(C.POINTER(C.c_double)), rows, C.byref(n)))
+    return out[:n.value].copy()
 
 
 def order_parameters(engine, slot):
