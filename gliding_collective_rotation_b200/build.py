@@ -18,7 +18,8 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgcr.so")
-SOURCES = ["gcr_step.cu", "gcr_lists.cu", "gcr_abi.cu", "gcr_noalloc.cu", "gcr_observables.cu"]
+SOURCES = ["gcr_step.cu", "gcr_steps_2d.cu", "gcr_steps_2f.cu", "gcr_steps_3d.cu", "gcr_steps_3f.cu", "gcr_lists.cu",
+           "gcr_abi.cu", "gcr_noalloc.cu", "gcr_observables.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden",
          "--expt-relaxed-constexpr"]

@@ -147,6 +147,7 @@ struct gcr_ctx {
     size_t pair_cells_smem = 0;
     size_t pair_smem = 0;
     size_t build_smem = 0;
+    size_t steps_smem = 0;
     int32_t *chain_starts = nullptr;
     void *corr = nullptr;  // scratch of the pair correlations (lazy): centres, angles, histograms
     size_t corr_bytes = 0;
@@ -164,6 +165,10 @@ struct gcr_ctx {
     int grid_update = 1, grid_sys = 1, grid_pair = 1, grid_bin = 1, grid_sort = 1, grid_build = 1;
     int grid_stage0 = 1, grid_stage1 = 1, grid_stage4[4] = {1, 1, 1, 1};
     int grid_stage0f = 1, grid_stage1f = 1, grid_pair_cells = 1;
+    TeamSync *team = nullptr;          // barrier state of the one-kernel steps
+    int grid_steps[3] = {-1, -1, -1};  // CTAs of them that fit at once, in clusters of kTeamCluster (-1: not asked)
+    int wide_steps[3] = {-1, -1, -1};  // a cluster of 16 CTAs fits
+    std::vector<int64_t> attempts;     // steps queued per slot since it was armed
     cudaGraphExec_t graph = nullptr;
     bool graph_rigid = false;  // the graph holds the rigid-rod projection kernels
     bool graph_obs = false;    // the graph holds the series kernel
@@ -187,6 +192,12 @@ namespace {
 // takes from the L1 cache: short lists (WCA) need few
 int build_cap(int block, int list_depth) { return std::min(list_depth <= 32 ? 12 : 32, 12288 / block); }
 
+// ... and in the one-kernel steps, where the CTAs of all tiles share the SMs
+constexpr int kTeamBuildCap = 24;
+
+// CTAs of a cluster of the one-kernel steps beyond one cluster
+constexpr int kTeamCluster = 8;
+
 int kernel_grid(const gcr_ctx *c, void *fn, int block, int64_t max_tiles, size_t smem = 0)
 {
     // ctas_per_sm < 0: one CTA per tile (the hardware scheduler streams the
@@ -198,6 +209,28 @@ int kernel_grid(const gcr_ctx *c, void *fn, int block, int64_t max_tiles, size_t
     int64_t g = (int64_t)c->sm_count * occ;
     g = std::min<int64_t>(g, std::max<int64_t>(max_tiles, 1));
     return (int)std::max<int64_t>(g, 1);
+}
+
+// clusters of n CTAs of a kernel that fit the device at once (0: none)
+int clusters_that_fit(const gcr_ctx *c, void *fn, int n, int block, size_t smem)
+{
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(n);
+    lc.blockDim = dim3(block);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = c->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = n;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, fn, &lc) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return clusters;
 }
 
 int rebuild_tiles(gcr_ctx *c)
@@ -686,10 +719,10 @@ int enqueue_step(gcr_ctx *c)
 // start of a run: flag the armed systems whose neighbour lists no longer
 // cover their positions (the host may have moved beads between calls); the
 // others keep their lists
-int enqueue_run_start(gcr_ctx *c)
+int enqueue_run_start(gcr_ctx *c, bool one_kernel)
 {
     int rc = launch(c, c->ks.run_check, c->grid_update, c->cfg.block_beads);
-    return rc ? rc : launch_duty(c, kDutyStart);
+    return rc || one_kernel ? rc : launch_duty(c, kDutyStart);
 }
 
 // a list build of `slot` before its next pair forces, from zeroed cell
@@ -737,6 +770,116 @@ int build_graph(gcr_ctx *c)
     e = cudaGraphInstantiate(&c->graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(GCR_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+    return GCR_OK;
+}
+
+// which k_steps a batch needs
+int steps_kind(const gcr_ctx *c)
+{
+    if (c->cfg.srk_order == 4) return 2;
+    for (size_t s = 0; s < c->slots.size(); s++)
+        if (c->slots[s].used && c->hP[s].grp_n > 0) return 1;
+    return any_rigid(c) ? 1 : 0;
+}
+
+// Steps run in one kernel (k_steps) while every tile has a CTA of its own, of
+// those that fit at once (592 of 128 threads); a second round would wait for
+// the first between two barriers.  One step, us, by launches and in one kernel
+// (B200): 1000 beads 28, 20; 4000 30, 26; 64,000 33, 32; four sweep systems of
+// 82,000 beads, two rounds, 37, 48; FP64 1000 31, 22; 32,000 39, 30.  Coupled
+// populations and SRK4 have more barriers a step and half the limit: motors
+// 15,000 beads 94, 81, 61,000 beads 137, 153; SRK4 1500 beads 63, 37.  One CTA
+// per tile (ctas_per_sm < 0) and the cell-staged pair forces always use
+// launches.
+bool one_kernel_steps(gcr_ctx *c)
+{
+    if (c->cfg.ctas_per_sm < 0 || c->cfg.pair_mode == 2) return false;
+    const int kind = steps_kind(c), bb = c->cfg.block_beads;
+    const int64_t tiles = (int64_t)c->h_bead_tiles.size();
+    // no more than the registers allow fit; a portable cluster always does
+    // (the device is asked only where that leaves it open: a query takes longer
+    // than a step)
+    if (tiles > (int64_t)c->sm_count * std::max(1, 65536 / (128 * bb))) return false;
+    void *fn = c->ks.steps[kind];
+    if (c->grid_steps[kind] < 0) {
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->steps_smem);
+        c->grid_steps[kind] = 0;
+    }
+    if (tiles <= kTeamCluster) return true;
+    if (tiles <= 16 && c->wide_steps[kind] < 0) {
+        const bool wide = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        if (!wide) (void)cudaGetLastError();
+        c->wide_steps[kind] = wide && clusters_that_fit(c, fn, 16, bb, c->steps_smem) > 0 ? 1 : 0;
+    }
+    if (tiles <= 16 && c->wide_steps[kind] > 0) return true;
+    if (c->grid_steps[kind] == 0) {
+        int64_t fit = (int64_t)clusters_that_fit(c, fn, kTeamCluster, bb, c->steps_smem) * kTeamCluster;
+        if (c->cfg.ctas_per_sm > 0) fit = std::min<int64_t>(fit, (int64_t)c->cfg.ctas_per_sm * c->sm_count);
+        c->grid_steps[kind] = std::max(1, (int)(fit - fit % kTeamCluster));
+    }
+    return tiles <= c->grid_steps[kind] / (kind == 0 ? 1 : 2);
+}
+
+// `steps` steps of every armed system in one kernel
+int launch_steps(gcr_ctx *c, int64_t steps)
+{
+    const int kind = steps_kind(c);
+    const int tiles = std::max<int>(1, (int)c->h_bead_tiles.size());
+    int n = (int)steps, motor = any_motor(c) ? 1 : 0, rigid = any_rigid(c) ? 1 : 0;
+    // a few tiles: one cluster of a power of two CTAs (those past the tiles
+    // only keep the barriers); else clusters of kTeamCluster
+    const bool one = tiles <= kTeamCluster || (tiles <= 16 && c->wide_steps[kind] > 0);
+    int csize = one ? 1 << ilog2(tiles) : kTeamCluster;
+    const int grid = one ? csize : (tiles + csize - 1) / csize * csize;
+    GCR_CUDA(cudaMemsetAsync(c->team, 0, sizeof(TeamSync), c->stream));
+    BatchArgs args = c->args;
+    args.build_cap = std::min(kTeamBuildCap, args.build_cap);
+    void *a[] = {&args, &c->team, &n, &csize, &motor, &rigid};
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(c->cfg.block_beads);
+    lc.dynamicSmemBytes = c->steps_smem;
+    lc.stream = c->stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = csize;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeCooperative;
+    at[1].val.cooperative = 1;
+    lc.attrs = at;
+    lc.numAttrs = one ? 1 : 2;
+    GCR_CUDA(cudaLaunchKernelExC(&lc, c->ks.steps[kind], a));
+    return GCR_OK;
+}
+
+// steps until some system's series takes its next row (at most `steps`):
+// its call's steps, plus the call's phase, reach a multiple of the interval
+int64_t steps_to_row(const gcr_ctx *c, int64_t steps)
+{
+    for (size_t s = 0; s < c->slots.size(); s++) {
+        const SysS &st = c->hS[s];
+        if (!c->slots[s].used || !st.series || st.series_every <= 0) continue;
+        const int64_t at = (c->attempts[s] + st.series_phase) % st.series_every;
+        steps = std::min(steps, st.series_every - at);
+    }
+    return steps;
+}
+
+// steps of one launch at most: a bound on the time a kernel holds the device
+constexpr int64_t kTeamSteps = 512;
+
+int run_one_kernel(gcr_ctx *c, int64_t steps)
+{
+    const bool obs = any_series(c);
+    while (steps > 0) {
+        int64_t n = std::min(steps, kTeamSteps);
+        if (obs) n = steps_to_row(c, n);
+        int rc = launch_steps(c, n);
+        if (!rc && obs) rc = launch_observe(c);
+        if (rc) return rc;
+        for (int64_t &q : c->attempts) q += n;
+        steps -= n;
+    }
     return GCR_OK;
 }
 
@@ -844,6 +987,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     e = e ? e : cudaMalloc(&c->img, sizeof(int) * (size_t)cfg.bead_capacity * cfg.dim);
     e = e ? e : cudaMalloc(&c->restb, sizeof(double) * (size_t)cfg.bead_capacity);
     e = e ? e : cudaMalloc(&c->work, sizeof(int) * (size_t)(3 + 3 * (S + 1)));
+    e = e ? e : cudaMalloc(&c->team, sizeof(TeamSync));
     e = e ? e : cudaMalloc(&c->xi, (size_t)cfg.bead_capacity * cfg.dim * (cfg.precision == GCR_FP64 ? 8 : 4));
     e = e ? e : cudaMalloc(&c->fp, (size_t)cfg.bead_capacity * cfg.dim * (cfg.precision == GCR_FP64 ? 8 : 4));
     e = e ? e : cudaMalloc(&c->chain_starts, sizeof(int32_t) * (cfg.bead_capacity + S));
@@ -865,6 +1009,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     c->slots.assign(S, Slot());
     c->hP.assign(S, SysP());
     c->hS.assign(S, SysS());
+    c->attempts.assign(S, 0);
     c->beads.init(cfg.bead_capacity);
     c->cells.init(cfg.cell_capacity);
     c->chains.init(cfg.bead_capacity + S);
@@ -930,6 +1075,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     c->grid_sort = kernel_grid(c, c->ks.sort, cfg.block_cells, c->max_cell_tiles);
     c->grid_build = kernel_grid(c, c->ks.build0, cfg.block_beads, c->max_bead_tiles, c->build_smem);
     c->grid_sys = (int)((S + 127) / 128);
+    c->steps_smem = std::max(c->pair_smem, sizeof(int) * (size_t)std::min(kTeamBuildCap, a.build_cap) * cfg.block_beads);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return cleanup(fail(GCR_ERR_CUDA, "initialisation"));
     *out = c;
     return GCR_OK;
@@ -942,7 +1088,7 @@ int gcr_destroy(gcr_ctx *c)
     if (c->graph) cudaGraphExecDestroy(c->graph);
     void *ptrs[] = {c->dP, c->dS, c->d_bead_tiles, c->d_cell_tiles, c->d_ntiles, c->d_row_prefix, c->topo, c->cnt[0],
                     c->cnt[1], c->items, c->nbr, c->ncount, c->xref, c->work, c->xi, c->fp, c->chain_starts, c->d_err,
-                    c->d_out, c->pos2, c->faux, c->xnbr, c->xcount, c->img, c->act, c->mpush, c->mdelta, c->restb, c->corr};
+                    c->d_out, c->pos2, c->faux, c->xnbr, c->xcount, c->img, c->act, c->mpush, c->mdelta, c->restb, c->corr, c->team};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -1333,8 +1479,10 @@ int gcr_call_begin_batch(gcr_ctx *c, int32_t n, const int32_t *slots, const gcr_
     GCR_CUDA(cudaMemcpyAsync(c->hS.data(), c->dS, sizeof(SysS) * S, cudaMemcpyDeviceToHost, c->stream));
     GCR_CUDA(cudaStreamSynchronize(c->stream));
     std::vector<int> stopped;
-    for (int i = 0; i < n; i++)
+    for (int i = 0; i < n; i++) {
         if (arm(c->hS[slots[i]], calls + i)) stopped.push_back(slots[i]);
+        c->attempts[slots[i]] = 0;
+    }
     GCR_CUDA(cudaMemcpyAsync(c->dS, c->hS.data(), sizeof(SysS) * S, cudaMemcpyHostToDevice, c->stream));
     for (int sl : stopped) {
         int rc = mark_rebuild(c, sl);
@@ -1354,6 +1502,7 @@ int gcr_call_begin(gcr_ctx *c, int32_t slot, const gcr_call *call)
     GCR_CUDA(cudaMemcpyAsync(&s, c->dS + slot, sizeof(SysS), cudaMemcpyDeviceToHost, c->stream));
     GCR_CUDA(cudaStreamSynchronize(c->stream));
     const bool stopped = arm(s, call);
+    c->attempts[slot] = 0;
     GCR_CUDA(cudaMemcpyAsync(c->dS + slot, &s, sizeof(SysS), cudaMemcpyHostToDevice, c->stream));
     if (stopped && (rc = mark_rebuild(c, slot))) return rc;
     GCR_CUDA(cudaStreamSynchronize(c->stream));
@@ -1368,14 +1517,21 @@ int gcr_run(gcr_ctx *c, int64_t max_steps, int32_t sync_every)
         int rc = rebuild_tiles(c);
         if (rc) return rc;
     }
-    int rc = build_graph(c);
+    const bool one_kernel = one_kernel_steps(c);
+    int rc = one_kernel ? GCR_OK : build_graph(c);
     if (rc) return rc;
-    rc = enqueue_run_start(c);
+    rc = enqueue_run_start(c, one_kernel);
     if (rc) return rc;
     const int64_t spg = c->cfg.steps_per_graph;
     const int64_t graphs = (max_steps + spg - 1) / spg;
+    if (one_kernel && sync_every <= 0) return run_one_kernel(c, graphs * spg);
     for (int64_t g = 0; g < graphs; g++) {
-        GCR_CUDA(cudaGraphLaunch(c->graph, c->stream));
+        if (one_kernel) {
+            if ((rc = run_one_kernel(c, spg))) return rc;
+        } else {
+            GCR_CUDA(cudaGraphLaunch(c->graph, c->stream));
+            for (int64_t &q : c->attempts) q += spg;
+        }
         if (sync_every > 0 && (g + 1) % sync_every == 0 && g + 1 < graphs) {
             int32_t n = 0;
             rc = gcr_count_active(c, &n);
@@ -1395,7 +1551,7 @@ int gcr_profile_steps(gcr_ctx *c, int32_t n_steps, float *ms_out)
         int rc = rebuild_tiles(c);
         if (rc) return rc;
     }
-    int rc = enqueue_run_start(c);
+    int rc = enqueue_run_start(c, false);
     if (rc) return rc;
     // groups: lists(pos), pair(pos), stage 0, lists(pos1), pair(pos1),
     // stage 1 + dt rule, update + bookkeeping
@@ -1404,6 +1560,7 @@ int gcr_profile_steps(gcr_ctx *c, int32_t n_steps, float *ms_out)
     for (auto &e : ev) GCR_CUDA(cudaEventCreate(&e));
     const int bb = c->cfg.block_beads;
     const bool rigid = any_rigid(c), cross = any_cross(c);
+    for (int64_t &q : c->attempts) q += n_steps;
     for (int s = 0; s < n_steps && rc == GCR_OK; s++) {
         cudaEvent_t *e = ev.data() + (size_t)s * (G + 1);
         GCR_CUDA(cudaEventRecord(e[0], c->stream));

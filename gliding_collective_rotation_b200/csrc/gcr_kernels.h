@@ -66,6 +66,14 @@ struct BatchArgs {
 // per-system work after a kernel or phase of the step (gcr_phases.cuh)
 enum { kDutyNone, kDutyStart, kDutyPlan, kDutyDt, kDutyEnd };
 
+// barrier state of the one-kernel steps, zeroed before each launch
+struct TeamSync {
+    unsigned long long arrived;  // asks for a list plan << 32 | clusters that reached a barrier, over all barriers
+    unsigned long long pad[31];  // the polled word apart from the counter
+    unsigned long long open;     // (last barrier opened << 34) | asks << 2 | outcome of its duty
+    unsigned long long pad2[31];
+};
+
 struct KernelSet {
     void *bin0;     // cell binning of pos / pos1 for a list build
     void *bin1;
@@ -94,6 +102,7 @@ struct KernelSet {
     void *pair_cross[3];  // pair forces at pos / pos1 / pos2 with the other populations' (coupled systems)
     void *pair_cells[2];  // cell-staged pair forces at pos / pos1 (pair_mode 2)
     void *motor[2];       // motor decisions of stage 0 / 1 (graphs with a motor population)
+    void *steps[3];       // whole steps in one kernel: SRK2 uncoupled, SRK2, SRK4
     size_t (*pair_cells_smem)(int cap);  // their dynamic shared memory for `cap` staged beads
     int pair_cells_rows;  // cell rows a row tile stages (3 in 2D, 9 in 3D)
     int max_row_cells;    // cells of a row tile, at most
@@ -101,6 +110,11 @@ struct KernelSet {
 };
 
 KernelSet kernel_set(int dim, int precision);
+// fill in `steps` (a translation unit each: they compile for a minute)
+void steps_kernels_2d(KernelSet &k);
+void steps_kernels_2f(KernelSet &k);
+void steps_kernels_3d(KernelSet &k);
+void steps_kernels_3f(KernelSet &k);
 
 // message returned by gcr_last_error() on the calling thread (gcr_abi.cu)
 void set_last_error(const char *msg);

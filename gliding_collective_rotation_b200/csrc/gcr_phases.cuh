@@ -263,11 +263,18 @@ __device__ __forceinline__ bool left_skin(const SysP &p, const BatchArgs &A, int
     return left_skin_of<D>(p, A.xref + (size_t)(p.bead_off + b) * D, x);
 }
 
-// the tiles a CTA works on: first, first + step, ...
+// the tiles a CTA works on: first, first + step, ...; the bead tiles there are
+// and the first one's table entry (read once for many steps by k_steps)
 struct Span {
-    int first, step;
+    int first, step, bead_tiles;
+    Tile tile;
 };
-__device__ __forceinline__ Span launch_span() { return Span{(int)blockIdx.x, (int)gridDim.x}; }
+__device__ __forceinline__ Span list_span() { return Span{(int)blockIdx.x, (int)gridDim.x, 0, Tile{0, 0}}; }
+__device__ __forceinline__ Span bead_span(const BatchArgs &A)
+{
+    const int nt = *A.n_bead_tiles, first = (int)blockIdx.x;
+    return Span{first, (int)gridDim.x, nt, first < nt ? A.bead_tiles[first] : Tile{0, 0}};
+}
 
 // Work list of a list build: the flagged systems, compacted, with the
 // running sum of their bead tiles and cell tiles.  Layout of A.work:
@@ -308,8 +315,9 @@ __device__ __forceinline__ int work_owner(const int *pre, int m, int i)
     return lo;
 }
 
-// one CTA: compact the systems that take part in a list build now
-static __device__ __noinline__ void plan_lists(const BatchArgs &A)
+// one CTA: compact the systems that take part in a list build now; returns
+// how many there are
+static __device__ __noinline__ int plan_lists(const BatchArgs &A)
 {
     __shared__ int sh[3][32];
     __shared__ int carry[3];
@@ -403,6 +411,26 @@ static __device__ __noinline__ void plan_lists(const BatchArgs &A)
         A.S[wsys[k]].rebuild = 0;
         A.S[wsys[k]].turn += 1;
     }
+    return carry[0];
+}
+
+// the dt of the largest force strength Sg, and the part of it that the call's
+// time limit leaves
+__device__ __forceinline__ double dt_of(double Sg, double dtmax, double mdps, double rk, const SysS &s, double &dt_used)
+{
+    double dt;
+    if (Sg == 0.0)
+        dt = dtmax;
+    else {
+        double q = mdps / Sg;
+        dt = (q < dtmax) ? q : dtmax;
+    }
+    dt_used = rk * dt;
+    if (s.max_dt_usable > 0.0) {
+        double lim = s.max_dt_usable - s.elapsed;
+        dt_used = (lim < dt_used) ? lim : dt_used;
+    }
+    return dt;
 }
 
 // per-system dt rule after stage 1 (SRK.py:323-353), of slot i
@@ -446,18 +474,8 @@ __device__ __forceinline__ void sys_dt(const BatchArgs &A, int i)
         s.flags |= group_fatal;
         return;
     }
-    double dt;
-    if (Sg == 0.0)
-        dt = dtmax;
-    else {
-        double q = mdps / Sg;
-        dt = (q < dtmax) ? q : dtmax;
-    }
-    double dt_used = rk * dt;
-    if (s.max_dt_usable > 0.0) {
-        double lim = s.max_dt_usable - s.elapsed;
-        dt_used = (lim < dt_used) ? lim : dt_used;
-    }
+    double dt_used;
+    const double dt = dt_of(Sg, dtmax, mdps, rk, s, dt_used);
     s.dt_next = dt;
     s.dt_used = dt_used;
     s.mfs = S;
@@ -468,11 +486,12 @@ __device__ __forceinline__ void sys_dt(const BatchArgs &A, int i)
 }
 
 // per-system step bookkeeping after the corrector (SRK.py:330, 348-349,
-// 128-130), of slot i; a step aborted by a fatal flag is not counted
-__device__ __forceinline__ void sys_end(const BatchArgs &A, int i)
+// 128-130), of slot i; a step aborted by a fatal flag is not counted.  True
+// while the system has more steps to take.
+__device__ __forceinline__ bool sys_end(const BatchArgs &A, int i)
 {
     SysS &s = A.S[i];
-    if (!s.active || (s.flags & kFlagFatal)) return;
+    if (!s.active || (s.flags & kFlagFatal)) return false;
     s.dt = s.dt_next;
     set_predictor(A.P[i], s, A.mixed);
     s.elapsed += s.dt_used;
@@ -482,6 +501,7 @@ __device__ __forceinline__ void sys_end(const BatchArgs &A, int i)
     bool more = (s.steps_done < s.max_steps || s.max_steps < 0) &&
                 (s.elapsed < s.max_dt_usable || s.max_dt_usable < 0.0);
     s.active = more ? 1 : 0;
+    return more;
 }
 
 // The per-system work between two kernels of a step, done by one CTA: the list
@@ -549,7 +569,7 @@ template <int D, int WHICH>
 __global__ void __launch_bounds__(512) k_bin(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
-    bin_tiles<D, WHICH>(A, launch_span());
+    bin_tiles<D, WHICH>(A, list_span());
 }
 
 // sort a cell's slot contents by bead id (the cell-staged pair forces sum in
@@ -855,7 +875,7 @@ template <int D, int WHICH>
 __global__ void __launch_bounds__(512, 2) k_build(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
-    build_tiles<D, WHICH>(A, launch_span());
+    build_tiles<D, WHICH>(A, list_span());
 }
 
 // pair forces between coupled populations: the force on bead b of one
@@ -1129,9 +1149,9 @@ __device__ __forceinline__ void pair_tiles(const BatchArgs &A, Span sp)
 {
     extern __shared__ __align__(16) unsigned char pair_smem[];
     FT *wbuf = reinterpret_cast<FT *>(pair_smem) + (size_t)(threadIdx.x >> 5) * (D + 1) * 32 * kPairChunk;
-    const int nt = *A.n_bead_tiles;
+    const int nt = sp.bead_tiles;
     // the next tile's table entry is loaded while the current tile runs
-    Tile nx = sp.first < nt ? A.bead_tiles[sp.first] : Tile{0, 0};
+    Tile nx = sp.tile;
     for (int t = sp.first; t < nt; t += sp.step) {
         const Tile tl = nx;
         if (t + sp.step < nt) nx = A.bead_tiles[t + sp.step];
@@ -1172,7 +1192,7 @@ template <int D, typename FT, int WHICH, bool CROSS>
 __global__ void __launch_bounds__(512, pair_min_blocks<D, FT>()) k_pair(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
-    pair_tiles<D, FT, WHICH, CROSS>(A, launch_span());
+    pair_tiles<D, FT, WHICH, CROSS>(A, bead_span(A));
 }
 
 // ------------------------------------------------------------------------
@@ -1482,16 +1502,17 @@ __device__ __forceinline__ void bond(const SysP &p, bool has, const double *x0, 
 }
 
 template <int D, typename FT, int STAGE, bool FUSED>
-__device__ __forceinline__ void stage_tiles(const BatchArgs &A, Span sp)
+__device__ __forceinline__ bool stage_tiles(const BatchArgs &A, Span sp)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using BT = typename Bonded<FT>::type;
     constexpr unsigned kAll = 0xffffffffu;
     constexpr uint8_t kInner = kHasPrev | kHasNext;
     const int lane = threadIdx.x & 31;
-    const int nt = *A.n_bead_tiles;
+    const int nt = sp.bead_tiles;
+    bool raised = false;  // this thread asked for a list build
     // the next tile's table entry is loaded while the current tile runs
-    Tile nx = sp.first < nt ? A.bead_tiles[sp.first] : Tile{0, 0};
+    Tile nx = sp.tile;
     for (int t = sp.first; t < nt; t += sp.step) {
         const Tile tl = nx;
         if (t + sp.step < nt) nx = A.bead_tiles[t + sp.step];
@@ -1794,7 +1815,7 @@ __device__ __forceinline__ void stage_tiles(const BatchArgs &A, Span sp)
                     if (!finite)
                         atomicOr(&s.flags, kFlagNonFinite);
                     else if (p.calc_wca && left_skin_of<D>(p, pre_r, x1))
-                        s.rebuild = 1;  // the list no longer covers the new positions
+                        s.rebuild = raised = true;  // the list no longer covers the new positions
                 }
             }
             if constexpr (STAGE == 1 || STAGE == 13) {
@@ -1819,13 +1840,14 @@ __device__ __forceinline__ void stage_tiles(const BatchArgs &A, Span sp)
             }
         }
     }
+    return raised;
 }
 
 template <int D, typename FT, int STAGE, bool FUSED = false>
 __global__ void __maxnreg__((stage_regs<D, FT>())) k_stage(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
-    stage_tiles<D, FT, STAGE, FUSED>(A, launch_span());
+    stage_tiles<D, FT, STAGE, FUSED>(A, bead_span(A));
 }
 
 // the update kernel holds all its inputs in registers at once
@@ -1838,12 +1860,16 @@ constexpr int update_min_blocks()
     return (D == 2 && sizeof(FT) == 4) ? GCR_UPDATE_MIN_BLOCKS : 1;
 }
 
-template <int D, typename FT>
-__device__ __forceinline__ void update_tiles(const BatchArgs &A, Span sp)
+// DT: the systems are not coupled, and each thread works out its system's dt
+// itself (the thread of bead 0 for the record), where a launch or a barrier
+// would cost more
+template <int D, typename FT, bool DT = false>
+__device__ __forceinline__ bool update_tiles(const BatchArgs &A, Span sp)
 {
-    const int nt = *A.n_bead_tiles;
+    const int nt = sp.bead_tiles;
+    bool raised = false;
     // the next tile's table entry is loaded while the current tile runs
-    Tile nx = sp.first < nt ? A.bead_tiles[sp.first] : Tile{0, 0};
+    Tile nx = sp.tile;
     for (int t = sp.first; t < nt; t += sp.step) {
         const Tile tl = nx;
         if (t + sp.step < nt) nx = A.bead_tiles[t + sp.step];
@@ -1881,8 +1907,26 @@ __device__ __forceinline__ void update_tiles(const BatchArgs &A, Span sp)
         }
         // no barriers in this kernel: a per-thread decision is safe
         if (!s.active || (s.flags & kFlagFatal) || !valid) continue;
-        const FT *sc = step_consts<FT>(s);
-        const FT dt_eff = sc[kSUpd], s2 = sc[kSUpdNoise];
+        FT dt_eff, s2, rot = FT(0);
+        if constexpr (DT) {
+            const double pref = A.order == 4 ? 1.0 : 0.5;
+            const double S = p.sqrt2D + pref * sqrt(__longlong_as_double((long long)s.max_f2)) / p.radius;
+            double dtu;
+            const double dt = dt_of(S, p.dtmax, p.mdps, p.rk, s, dtu);
+            dt_eff = (FT)(dtu * pref / p.radius);
+            s2 = (FT)sqrt(2.0 * dtu * p.D);
+            if (p.Dr > 0.0 && !p.get_orient) rot = (FT)(sqrt(2.0 * dtu * p.Dr) * 3.141592653589793);
+            if (b == 0) {
+                s.dt_next = dt;
+                s.dt_used = dtu;
+                s.mfs = S;
+            }
+        } else {
+            const FT *sc = step_consts<FT>(s);
+            dt_eff = sc[kSUpd];
+            s2 = sc[kSUpdNoise];
+            rot = sc[kSUpdRot];
+        }
         double x[3] = {0.0, 0.0, 0.0};
         bool finite = true;
         // an attached motor keeps its position (SRK.py:389-395)
@@ -1911,7 +1955,7 @@ __device__ __forceinline__ void update_tiles(const BatchArgs &A, Span sp)
             FT tb[3];
 #pragma unroll
             for (int i = 0; i < D; i++) tb[i] = tan[(size_t)b * D + i];
-            const FT sq = sc[kSUpdRot];
+            const FT sq = rot;
             FT proj = FT(0);
 #pragma unroll
             for (int i = 0; i < D; i++) proj += xr[i] * tb[i];
@@ -1928,15 +1972,17 @@ __device__ __forceinline__ void update_tiles(const BatchArgs &A, Span sp)
 #pragma unroll
             for (int i = 0; i < D; i++) tan[(size_t)b * D + i] = tb[i] / mag;
         }
-        if (plain && finite && p.calc_wca && left_skin_of<D>(p, xr, x)) s.rebuild = 1;  // rebuild before the next step
+        if (plain && finite && p.calc_wca && left_skin_of<D>(p, xr, x))
+            s.rebuild = raised = true;  // rebuild before the next step
     }
+    return raised;
 }
 
 template <int D, typename FT>
 __global__ void __launch_bounds__(512, update_min_blocks<D, FT>()) k_update(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
-    update_tiles<D, FT>(A, launch_span());
+    update_tiles<D, FT>(A, bead_span(A));
 }
 
 // ------------------------------------------------------------------------
@@ -1974,9 +2020,10 @@ __device__ __forceinline__ double wrap_open(double sep, double half, double L)
 }
 
 template <int D, typename FT, int STAGE>
-__device__ __forceinline__ void rigid_tiles(const BatchArgs &A, Span sp)
+__device__ __forceinline__ bool rigid_tiles(const BatchArgs &A, Span sp)
 {
-    const int nt = *A.n_bead_tiles;
+    const int nt = sp.bead_tiles;
+    bool raised = false;
     for (int t = sp.first; t < nt; t += sp.step) {
         const Tile tl = A.bead_tiles[t];
         const SysP &p = A.P[tl.sys];
@@ -2094,15 +2141,16 @@ __device__ __forceinline__ void rigid_tiles(const BatchArgs &A, Span sp)
             if (finite && p.calc_wca && left_skin<D>(p, A, b, x)) moved = true;
         }
         if (!finite) atomicOr(&s.flags, kFlagNonFinite);
-        if (moved) s.rebuild = 1;  // the list no longer covers the new positions
+        if (moved) s.rebuild = raised = true;  // the list no longer covers the new positions
     }
+    return raised;
 }
 
 template <int D, typename FT, int STAGE>
 __global__ void __launch_bounds__(512) k_rigid(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
-    rigid_tiles<D, FT, STAGE>(A, launch_span());
+    rigid_tiles<D, FT, STAGE>(A, bead_span(A));
 }
 
 // start of a run: the rest length of every armed bead's chain into restb;
@@ -2163,7 +2211,7 @@ __global__ void __launch_bounds__(512) k_run_check(const __grid_constant__ Batch
 template <int D, int WHICH>
 __device__ __forceinline__ void motor_tiles(const BatchArgs &A, Span sp)
 {
-    const int nt = *A.n_bead_tiles;
+    const int nt = sp.bead_tiles;
     for (int t = sp.first; t < nt; t += sp.step) {
         const Tile tl = A.bead_tiles[t];
         const SysP &p = A.P[tl.sys];
@@ -2242,7 +2290,227 @@ template <int D, int WHICH>
 __global__ void __launch_bounds__(512) k_motor(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
-    motor_tiles<D, WHICH>(A, launch_span());
+    motor_tiles<D, WHICH>(A, bead_span(A));
+}
+
+// ------------------------------------------------------------------------
+// whole steps in one kernel.  A step of a small batch is bound by its
+// launches: twelve or ten kernels of 2 to 8 us each, most of them list
+// kernels that find nothing to build.  Here one team of CTAs, all resident at
+// once, takes `steps` steps with the same phases in the same order, and the
+// launch boundaries become team barriers.  The per-system work between
+// phases (list plan, step bookkeeping) is done by one CTA while the others
+// wait, and only when there is some: a step has three barriers unless a list
+// is built.
+// A team of up to 16 CTAs is one thread-block cluster and meets at its
+// hardware barrier.  A larger one is a cooperative launch of clusters that
+// meet at a counter in global memory; every wait there is bounded: a CTA
+// that gives up stops every system (kFlagListCorrupt) and the team returns.
+// KIND: 0 SRK2 of uncoupled systems without the rigid-rod projection (the
+// stage sums its pair forces itself); 1 every SRK2 batch; 2 every SRK4 batch.
+// ------------------------------------------------------------------------
+constexpr unsigned kTeamLists = 1, kTeamStop = 2;
+// polls before a waiting CTA gives up: each takes some hundred ns, the longest
+// phase a few ms
+constexpr int kTeamPolls = 1 << 23;
+
+// one CTA: a duty between two phases; ask: some thread asked for a list build
+// since the last plan
+static __device__ __noinline__ unsigned team_duty(const BatchArgs &A, int duty, bool ask)
+{
+    if (duty == kDutyDt) {
+        for (int i = threadIdx.x; i < A.n_slots; i += blockDim.x) sys_dt(A, i);
+        return 0;
+    }
+    if (duty == kDutyStart) {
+        step_duty(A, kDutyStart);
+        __syncthreads();
+        return A.work[0] > 0 ? kTeamLists : 0;
+    }
+    if (duty == kDutyEnd) {
+        bool more = false;
+        for (int i = threadIdx.x; i < A.n_slots; i += blockDim.x) more |= sys_end(A, i);
+        if (!__syncthreads_or(more)) return kTeamStop;
+    }
+    return ask && plan_lists(A) > 0 ? kTeamLists : 0;
+}
+
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// a word of another CTA of the cluster, at the same place of its shared memory
+__device__ __forceinline__ void store_cluster(unsigned *q, int rank, unsigned v)
+{
+    const unsigned a = (unsigned)__cvta_generic_to_shared(q);
+    asm volatile("{\n\t.reg .u32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\tst.shared::cluster.u32 [r], %2;\n\t}" ::"r"(a),
+                 "r"(rank), "r"(v)
+                 : "memory");
+}
+
+struct Team {
+    TeamSync *ts;
+    unsigned round;  // barriers passed
+    unsigned asks;   // asks for a plan up to the last barrier (a cluster's first thread)
+    int csize;       // CTAs of a cluster
+
+    // All CTAs of the team meet; raised: the thread asked for a list build.
+    // Returns the outcome of the duty.  The CTAs of a cluster tell one another
+    // through their shared memory (two sets of words in turn, so that none is
+    // overwritten before it is read) and one of them stands for the cluster at
+    // the counter.
+    __device__ __forceinline__ unsigned sync(const BatchArgs &A, int duty, bool raised = false)
+    {
+        __shared__ unsigned sh_word[2][17];  // asks of the cluster's CTAs, outcome
+        __shared__ int sh_last;
+        round++;
+        unsigned *word = sh_word[round & 1];
+        const int rank = blockIdx.x % csize, lane = threadIdx.x & 31;
+        bool ask = __syncthreads_or(raised);
+        if ((int)threadIdx.x < csize) store_cluster(word + rank, threadIdx.x, ask);
+        cluster_sync();
+        ask = __any_sync(0xffffffffu, lane < csize && word[lane < 16 ? lane : 0] != 0);
+        const bool whole = (int)gridDim.x == csize;
+        const bool idle = duty == kDutyNone || (duty == kDutyPlan && !ask);
+        if (whole && idle) return 0;
+        if (rank == 0) {
+            unsigned info = 0;
+            if (whole) {
+                info = team_duty(A, duty, ask);
+            } else {
+                __shared__ unsigned sh_info;
+                if (threadIdx.x == 0) {
+                    unsigned long long old, add = 1ull + ((unsigned long long)ask << 32);
+                    asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], %2;"
+                                 : "=l"(old)
+                                 : "l"(&ts->arrived), "l"(add)
+                                 : "memory");
+                    sh_last = ((unsigned)old + 1u) * csize == round * gridDim.x;
+                    const unsigned now = (unsigned)(old >> 32) + ask;
+                    sh_info = now != asks;
+                    if (sh_last) asks = now;
+                }
+                __syncthreads();
+                if (sh_last) {
+                    const bool any = sh_info;
+                    if (duty != kDutyNone && (duty != kDutyPlan || any)) info = team_duty(A, duty, any);
+                    __syncthreads();
+                    if (threadIdx.x == 0) {
+                        const unsigned long long v =
+                            (unsigned long long)(round & 0x3fffffffu) << 34 | (unsigned long long)asks << 2 | info;
+                        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(&ts->open), "l"(v) : "memory");
+                        sh_info = info;
+                    }
+                } else if (threadIdx.x == 0) {
+                    unsigned long long v = 0;
+                    int polls = 0;
+                    do {
+                        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&ts->open) : "memory");
+                    } while ((unsigned)(v >> 34) != (round & 0x3fffffffu) && ++polls < kTeamPolls);
+                    asks = (unsigned)(v >> 2);
+                    sh_info = (unsigned)v & 3u;
+                    if ((unsigned)(v >> 34) != (round & 0x3fffffffu)) {
+                        for (int i = 0; i < A.n_slots; i++) atomicOr(&A.S[i].flags, kFlagListCorrupt);
+                        sh_info = kTeamStop;
+                    }
+                }
+                __syncthreads();
+                info = sh_info;
+            }
+            if ((int)threadIdx.x < csize) store_cluster(word + 16, threadIdx.x, info);
+        }
+        cluster_sync();
+        return word[16];
+    }
+};
+
+// one stage's neighbour lists, for the systems the plan took
+template <int D, int WHICH>
+__device__ __forceinline__ bool team_lists(const BatchArgs &A, Team &team, Span sp)
+{
+    bin_tiles<D, WHICH>(A, sp);
+    if (team.sync(A, kDutyNone) & kTeamStop) return false;
+    build_tiles<D, WHICH>(A, sp);
+    if (team.sync(A, kDutyNone) & kTeamStop) return false;
+    // the plan has been carried out
+    if (blockIdx.x == 0 && threadIdx.x < 3) A.work[threadIdx.x] = 0;
+    return true;
+}
+
+// pair forces, motors and stage S of a batch of any kind; false: the team stops
+template <int D, typename FT, int S>
+__device__ __forceinline__ bool team_stage(const BatchArgs &A, Team &team, Span sp, bool motor, bool rigid,
+                                           bool &raised)
+{
+    constexpr int W = stage_reads(S);
+    pair_tiles<D, FT, W, true>(A, sp);
+    if constexpr (!srk4_stage(S)) {
+        if (motor) {
+            motor_tiles<D, S>(A, sp);
+            if (team.sync(A, kDutyNone) & kTeamStop) return false;
+        }
+    }
+    raised = stage_tiles<D, FT, S, false>(A, sp);
+    if constexpr (stage_writes(S) != 0) {
+        if (rigid) {
+            if (team.sync(A, kDutyNone) & kTeamStop) return false;
+            raised |= rigid_tiles<D, FT, S>(A, sp);
+        }
+    }
+    return true;
+}
+
+template <int D, typename FT, int KIND>
+__global__ void __maxnreg__(128)
+    k_steps(const __grid_constant__ BatchArgs A, TeamSync *ts, int steps, int csize, int motor, int rigid)
+{
+    Team team{ts, 0, 0, csize};
+    const Span sp = bead_span(A);
+    unsigned info = team.sync(A, kDutyStart);
+    bool raised = false;
+    for (int k = 0; k < steps; k++) {
+        if ((info & kTeamLists) && !team_lists<D, 0>(A, team, sp)) return;
+        if constexpr (KIND == 2) {
+            if (!team_stage<D, FT, 10>(A, team, sp, false, rigid, raised)) return;
+            info = team.sync(A, kDutyPlan, raised);
+            if (info & kTeamStop) return;
+            if ((info & kTeamLists) && !team_lists<D, 1>(A, team, sp)) return;
+            if (!team_stage<D, FT, 11>(A, team, sp, false, rigid, raised)) return;
+            info = team.sync(A, kDutyPlan, raised);
+            if (info & kTeamStop) return;
+            if ((info & kTeamLists) && !team_lists<D, 2>(A, team, sp)) return;
+            if (!team_stage<D, FT, 12>(A, team, sp, false, rigid, raised)) return;
+            info = team.sync(A, kDutyPlan, raised);
+            if (info & kTeamStop) return;
+            if ((info & kTeamLists) && !team_lists<D, 1>(A, team, sp)) return;
+            if (!team_stage<D, FT, 13>(A, team, sp, false, false, raised)) return;
+        } else {
+            if constexpr (KIND == 1) {
+                if (!team_stage<D, FT, 0>(A, team, sp, motor, rigid, raised)) return;
+            } else {
+                raised = stage_tiles<D, FT, 0, true>(A, sp);
+            }
+            info = team.sync(A, kDutyPlan, raised);
+            if (info & kTeamStop) return;
+            if ((info & kTeamLists) && !team_lists<D, 1>(A, team, sp)) return;
+            if constexpr (KIND == 1) {
+                if (!team_stage<D, FT, 1>(A, team, sp, motor, false, raised)) return;
+            } else {
+                stage_tiles<D, FT, 1, true>(A, sp);
+            }
+        }
+        if (team.sync(A, KIND == 0 ? kDutyNone : kDutyDt) & kTeamStop) return;
+        raised = update_tiles<D, FT, KIND == 0>(A, sp);
+        if constexpr (KIND != 0) {
+            if (rigid) {
+                if (team.sync(A, kDutyNone) & kTeamStop) return;
+                raised |= rigid_tiles<D, FT, KIND == 2 ? 13 : 1>(A, sp);
+            }
+        }
+        info = team.sync(A, kDutyEnd, raised);
+        if (info & kTeamStop) return;
+    }
 }
 
 }  // namespace gcr

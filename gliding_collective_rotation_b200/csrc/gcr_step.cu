@@ -14,7 +14,7 @@ __global__ void __launch_bounds__(1024) k_duty(const __grid_constant__ BatchArgs
 __global__ void __launch_bounds__(512) k_sort(const __grid_constant__ BatchArgs A)
 {
     pdl_wait();
-    sort_tiles(A, launch_span());
+    sort_tiles(A, list_span());
 }
 
 // chain-neighbour bits of every bead of one system
@@ -76,6 +76,10 @@ struct StepKernels {
 KernelSet kernel_set(int dim, int precision)
 {
     KernelSet k{};
+    if (dim == 2)
+        precision == 0 ? steps_kernels_2d(k) : steps_kernels_2f(k);
+    else
+        precision == 0 ? steps_kernels_3d(k) : steps_kernels_3f(k);
     if (dim == 2)
         k.pair_smem = precision == 0 ? pair_smem_bytes<2, double> : pair_smem_bytes<2, float>;
     else
