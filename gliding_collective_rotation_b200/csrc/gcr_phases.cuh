@@ -1006,12 +1006,21 @@ __device__ __forceinline__ void pair_term(const SysP &p, const double *xj, const
 constexpr int kRowBusy = GCR_PAIR_ROW_BUSY;
 // Partners in flight in a walked row.  3D lists are long and their gathers
 // miss: four take the pair kernel of a million LJ beads from 155 to 135 us.
-// In 2D mixed precision they cost registers and gain nothing (500k LJ beads 79
-// against 80 us).
+// In 2D they cost registers and gain nothing (500k LJ beads 79 against 80 us,
+// the 64-system sweep in FP64 44 against 46), except where a batch is small
+// enough for latency to bound it (k_steps).
 template <int D>
 constexpr int row_ahead()
 {
     return D == 3 ? 4 : 1;
+}
+// ... in k_steps: eight in 2D (40 steps of 10,000 LJ beads 2185 -> 1896 us, of
+// 37,000 in FP64 2576 -> 2432; walking rows of fewer busy lanes too was slower
+// once the chains had condensed)
+template <int D>
+constexpr int team_row_ahead()
+{
+    return D == 3 ? 4 : 8;
 }
 
 template <int D, typename FT>
@@ -1020,12 +1029,12 @@ size_t pair_smem_bytes(int TB)
     return (size_t)(TB / 32) * (D + 1) * 32 * kPairChunk * sizeof(FT);
 }
 
-template <int D, typename FT>
+template <int D, typename FT, int U>
 __device__ __forceinline__ void warp_list_pair_force(const BatchArgs &A, const SysP &p, const double *X,
                                                      const double *xb, int b, int cnt, FT *F, bool &bad, FT *buf)
 {
     constexpr unsigned kAll = 0xffffffffu;
-    constexpr int C = kPairChunk, Q = 32 * C, U = row_ahead<D>();
+    constexpr int C = kPairChunk, Q = 32 * C;
     const int lane = threadIdx.x & 31;
     cnt = cnt < 0 ? 0 : (cnt < A.list_depth ? cnt : A.list_depth);
     const int n = p.n;
@@ -1176,7 +1185,7 @@ __device__ __forceinline__ void pair_tiles(const BatchArgs &A, Span sp)
         bool bad = false;
         // motors have no pair force of their own (their zero-strength WCA
         // only bins them) and no list of one another
-        warp_list_pair_force<D, FT>(A, p, X, xb, b, valid && !p.motor ? cnt : 0, F, bad, wbuf);
+        warp_list_pair_force<D, FT, row_ahead<D>()>(A, p, X, xb, b, valid && !p.motor ? cnt : 0, F, bad, wbuf);
         // a motor's cross list is its candidate beads, not a force
         if constexpr (CROSS)
             if (valid && !p.motor) add_cross<D, FT, WHICH>(A, p, b, xb, F, bad);
@@ -1501,7 +1510,8 @@ __device__ __forceinline__ void bond(const SysP &p, bool has, const double *x0, 
     }
 }
 
-template <int D, typename FT, int STAGE, bool FUSED>
+// U: partners in flight in a walked row
+template <int D, typename FT, int STAGE, bool FUSED, int U = row_ahead<D>()>
 __device__ __forceinline__ bool stage_tiles(const BatchArgs &A, Span sp)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1696,9 +1706,9 @@ __device__ __forceinline__ bool stage_tiles(const BatchArgs &A, Span sp)
         if constexpr (FUSED) {
             __syncwarp();
             bool bad = false;
-            warp_list_pair_force<D, FT>(A, p, X, xb, b, cnt, Fp, bad,
-                                        reinterpret_cast<FT *>(smem_raw) +
-                                            (size_t)(threadIdx.x >> 5) * (D + 1) * 32 * kPairChunk);
+            warp_list_pair_force<D, FT, U>(A, p, X, xb, b, cnt, Fp, bad,
+                                           reinterpret_cast<FT *>(smem_raw) +
+                                               (size_t)(threadIdx.x >> 5) * (D + 1) * 32 * kPairChunk);
             if (bad) atomicOr(&s.flags, kFlagListCorrupt);
         }
         double mf2 = 0.0;
@@ -2489,7 +2499,7 @@ __global__ void __maxnreg__(128)
             if constexpr (KIND == 1) {
                 if (!team_stage<D, FT, 0>(A, team, sp, motor, rigid, raised)) return;
             } else {
-                raised = stage_tiles<D, FT, 0, true>(A, sp);
+                raised = stage_tiles<D, FT, 0, true, team_row_ahead<D>()>(A, sp);
             }
             info = team.sync(A, kDutyPlan, raised);
             if (info & kTeamStop) return;
@@ -2497,7 +2507,7 @@ __global__ void __maxnreg__(128)
             if constexpr (KIND == 1) {
                 if (!team_stage<D, FT, 1>(A, team, sp, motor, false, raised)) return;
             } else {
-                stage_tiles<D, FT, 1, true>(A, sp);
+                stage_tiles<D, FT, 1, true, team_row_ahead<D>()>(A, sp);
             }
         }
         if (team.sync(A, KIND == 0 ? kDutyNone : kDutyDt) & kTeamStop) return;
