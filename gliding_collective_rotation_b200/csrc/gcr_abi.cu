@@ -163,8 +163,8 @@ struct gcr_ctx {
     RangeAlloc beads, cells, chains;
     BatchArgs args{};
     int grid_update = 1, grid_sys = 1, grid_pair = 1, grid_bin = 1, grid_sort = 1, grid_build = 1;
-    int grid_stage0 = 1, grid_stage1 = 1, grid_stage4[4] = {1, 1, 1, 1};
-    int grid_stage0f = 1, grid_stage1f = 1, grid_pair_cells = 1;
+    int grid_stage[6] = {}, grid_stage_own[6] = {};
+    int grid_pair_cells = 1;
     TeamSync *team = nullptr;          // barrier state of the one-kernel steps
     int grid_steps[3] = {-1, -1, -1};  // CTAs of them that fit at once, in clusters of kTeamCluster (-1: not asked)
     int wide_steps[3] = {-1, -1, -1};  // a cluster of 16 CTAs fits
@@ -632,6 +632,9 @@ int launch_observe(gcr_ctx *c)
     return launch_args(c, c->observe, (int)c->slots.size(), 1024, 0, a);
 }
 
+bool own_pair(const gcr_ctx *c, bool cross);
+int launch_stage(gcr_ctx *c, int k, bool cross);
+
 // one SRK4 step (SRK.py:166-215): four force evaluations at pos, pos1, pos2,
 // pos1, each with its lists; the virtual updates alternate pos1 / pos2
 int enqueue_step4(gcr_ctx *c)
@@ -643,8 +646,8 @@ int enqueue_step4(gcr_ctx *c)
         if ((rc = enqueue_lists(c, reads[k]))) return rc;
         void *pair = c->graph_cross ? c->ks.pair_cross[reads[k]]
                                     : (reads[k] == 0 ? c->ks.pair0 : (reads[k] == 1 ? c->ks.pair1 : c->ks.pair2));
-        if ((rc = launch(c, pair, c->grid_pair, bb, c->pair_smem))) return rc;
-        if ((rc = launch(c, c->ks.stage4[k], c->grid_stage4[k], bb))) return rc;
+        if (!own_pair(c, c->graph_cross) && (rc = launch(c, pair, c->grid_pair, bb, c->pair_smem))) return rc;
+        if ((rc = launch_stage(c, 2 + k, c->graph_cross))) return rc;
         if (k < 3 && c->graph_rigid && (rc = launch(c, c->ks.rigid4[k], c->grid_update, bb))) return rc;
         if ((rc = launch_duty(c, k < 3 ? kDutyPlan : kDutyDt))) return rc;
     }
@@ -654,24 +657,34 @@ int enqueue_step4(gcr_ctx *c)
     return c->graph_obs ? launch_observe(c) : GCR_OK;
 }
 
-// pair_mode of an SRK2 graph: 1 and 2 only without coupled populations,
+// pair_mode of a graph: 1 and 2 are SRK2 options without coupled populations,
 // whose cross forces only k_pair adds
 int pair_mode(const gcr_ctx *c, bool cross) { return (c->cfg.srk_order == 2 && !cross) ? c->cfg.pair_mode : 0; }
+
 // The stages walk the lists themselves (pair_mode 1, the same bits as 0) in 2D
-// mixed precision whatever the mode: the sweep's step takes 656 us so, 678
-// with the pair kernel.  Elsewhere only when asked for: in FP64 the 64-system
+// mixed precision whatever the mode: the sweep's step takes 645 us so, 678 with
+// the pair kernel, 16 SRK4 systems 145 against 155.  Elsewhere only when asked for: in FP64 the 64-system
 // sweep's two stages take 233 us so, 224 with the pair kernel (registers), and
 // 3D lists are long (505 against 377 us).
-bool fused_pair(const gcr_ctx *c, bool cross)
+bool own_pair(const gcr_ctx *c, bool cross)
 {
-    if (c->cfg.srk_order != 2 || cross || c->cfg.pair_mode == 2) return false;
-    return c->cfg.pair_mode == 1 || (c->cfg.dim == 2 && c->cfg.precision == GCR_MIXED);
+    if (cross) return false;
+    if (c->cfg.dim == 2 && c->cfg.precision == GCR_MIXED) return pair_mode(c, cross) != 2;
+    return pair_mode(c, cross) == 1;
+}
+
+// stage k: 0 predictor, 1 corrector, 2..5 SRK4
+int launch_stage(gcr_ctx *c, int k, bool cross)
+{
+    const bool own = own_pair(c, cross);
+    return launch(c, own ? c->ks.stage_own[k] : c->ks.stage[k], own ? c->grid_stage_own[k] : c->grid_stage[k],
+                  c->cfg.block_beads, own ? c->pair_smem : 0);
 }
 
 // SRK2 stage s (0 predictor, 1 corrector): the pair forces, then the stage
 int enqueue_pair(gcr_ctx *c, int s, bool cross)
 {
-    if (fused_pair(c, cross)) return GCR_OK;
+    if (own_pair(c, cross)) return GCR_OK;
     if (pair_mode(c, cross) == 2) return launch(c, c->ks.pair_cells[s], c->grid_pair_cells, c->cfg.block_beads, c->pair_cells_smem);
     void *pair = cross ? c->ks.pair_cross[s] : (s == 0 ? c->ks.pair0 : c->ks.pair1);
     return launch(c, pair, c->grid_pair, c->cfg.block_beads, c->pair_smem);
@@ -681,11 +694,8 @@ int enqueue_pair(gcr_ctx *c, int s, bool cross)
 // after the predictor
 int enqueue_stage(gcr_ctx *c, int s, bool cross, bool rigid)
 {
-    const bool f = fused_pair(c, cross);
-    void *stage = s == 0 ? (f ? c->ks.stage0f : c->ks.stage0) : (f ? c->ks.stage1f : c->ks.stage1);
-    const int grid = s == 0 ? (f ? c->grid_stage0f : c->grid_stage0) : (f ? c->grid_stage1f : c->grid_stage1);
     const int bb = c->cfg.block_beads;
-    int rc = launch(c, stage, grid, bb, f ? c->pair_smem : 0);
+    int rc = launch_stage(c, s, cross);
     if (!rc && s == 0 && rigid) rc = launch(c, c->ks.rigid0, c->grid_update, bb);
     return rc ? rc : launch_duty(c, s == 0 ? kDutyPlan : kDutyDt);
 }
@@ -1051,14 +1061,16 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     c->pair_smem = c->ks.pair_smem(cfg.block_beads);
     if (c->pair_smem > 48 * 1024)
         for (void *fn : {c->ks.pair0, c->ks.pair1, c->ks.pair2, c->ks.pair_cross[0], c->ks.pair_cross[1],
-                         c->ks.pair_cross[2], c->ks.stage0f, c->ks.stage1f})
+                         c->ks.pair_cross[2]})
             cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->pair_smem);
-    for (int k = 0; k < 4; k++)
-        c->grid_stage4[k] = kernel_grid(c, c->ks.stage4[k], cfg.block_beads, c->max_bead_tiles);
-    c->grid_stage0 = kernel_grid(c, c->ks.stage0, cfg.block_beads, c->max_bead_tiles);
-    c->grid_stage1 = kernel_grid(c, c->ks.stage1, cfg.block_beads, c->max_bead_tiles);
-    c->grid_stage0f = kernel_grid(c, c->ks.stage0f, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
-    c->grid_stage1f = kernel_grid(c, c->ks.stage1f, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
+    for (int k = 0; k < 6; k++) {
+        c->grid_stage[k] = kernel_grid(c, c->ks.stage[k], cfg.block_beads, c->max_bead_tiles);
+        void *fn = c->ks.stage_own[k];
+        if (!fn) continue;
+        if (c->pair_smem > 48 * 1024)
+            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->pair_smem);
+        c->grid_stage_own[k] = kernel_grid(c, fn, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
+    }
     c->pair_cells_smem = c->ks.pair_cells_smem(a.cell_stage_cap);
     if (c->pair_cells_smem > 48 * 1024)
         for (int k = 0; k < 2; k++)

@@ -82,18 +82,18 @@ struct KernelSet {
     void *build1;
     void *pair0;    // pair forces at pos / pos1
     void *pair1;
-    void *stage0;
-    void *stage1;
-    void *stage0f;  // stages 0 and 1 that sum the pair forces themselves (no k_pair launch)
-    void *stage1f;
+    // stages 0, 1 and SRK4's four; stage_own: those that sum the pair forces
+    // themselves (no k_pair launch; null where the pair kernel is always the
+    // faster)
+    void *stage[6];
+    void *stage_own[6];
     void *update;
     void *rigid0;   // rigid-rod projection: predictor (pos -> pos1) and corrector (pos1 -> pos)
     void *rigid1;
-    // SRK4: lists and pair forces at pos2, the four stages, their projections
+    // SRK4: lists and pair forces at pos2, the stages' projections
     void *bin2;
     void *build2;
     void *pair2;
-    void *stage4[4];
     void *rigid4[4];
     void *topo;
     void *duty;      // per-system work between two kernels of a step (kDuty...), one CTA

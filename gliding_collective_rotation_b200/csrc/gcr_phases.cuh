@@ -1467,8 +1467,9 @@ __device__ __forceinline__ double srk_update(double x, FT dt_eff, FT s2, FT f, F
 // stage and update kernels.  FUSED: the stage walks its beads' neighbour
 // lists itself (warp_list_pair_force, the same sums as k_pair) instead of
 // reading fp, which saves the pair kernel's launch, its second read of the
-// positions and the fp round trip (SRK2 without coupled populations only;
-// gcr_config.pair_mode 1, and 2D mixed precision).
+// positions and the fp round trip (gcr_config.pair_mode 1, and 2D mixed
+// precision; not with coupled populations, where it gains nothing: 128 boxes
+// of two, both stages 234 us either way).
 // Bound by issue and by the latency of dependent loads.  A warp works on its
 // own: with the bonds and bends staged in shared memory, four CTA barriers a
 // tile and a division, a square root and a dozen conversions of constants in

@@ -47,22 +47,33 @@ template <int D, typename FT>
 struct StepKernels {
     static void *pair0() { return (void *)k_pair<D, FT, 0, false>; }
     static void *pair1() { return (void *)k_pair<D, FT, 1, false>; }
-    static void *stage0() { return (void *)k_stage<D, FT, 0>; }
-    static void *stage1() { return (void *)k_stage<D, FT, 1>; }
-    static void *stage0f() { return (void *)k_stage<D, FT, 0, true>; }
-    static void *stage1f() { return (void *)k_stage<D, FT, 1, true>; }
     static void *pair_cells0() { return (void *)k_pair_cells<D, FT, 0>; }
     static void *pair_cells1() { return (void *)k_pair_cells<D, FT, 1>; }
     static void *update() { return (void *)k_update<D, FT>; }
     static void *rigid0() { return (void *)k_rigid<D, FT, 0>; }
     static void *rigid1() { return (void *)k_rigid<D, FT, 1>; }
+    // stages 0, 1 and 10..13 (SRK4), with the pair forces of k_pair or their own
+    static void fill_stages(KernelSet &k)
+    {
+        k.stage[0] = (void *)k_stage<D, FT, 0>;
+        k.stage[1] = (void *)k_stage<D, FT, 1>;
+        k.stage_own[0] = (void *)k_stage<D, FT, 0, true>;
+        k.stage_own[1] = (void *)k_stage<D, FT, 1, true>;
+        // SRK4: with their own in 2D mixed precision, else (and coupled) k_pair's
+        k.stage[2] = (void *)k_stage<D, FT, 10>;
+        k.stage[3] = (void *)k_stage<D, FT, 11>;
+        k.stage[4] = (void *)k_stage<D, FT, 12>;
+        k.stage[5] = (void *)k_stage<D, FT, 13>;
+        if constexpr (D == 2 && sizeof(FT) == 4) {
+            k.stage_own[2] = (void *)k_stage<D, FT, 10, true>;
+            k.stage_own[3] = (void *)k_stage<D, FT, 11, true>;
+            k.stage_own[4] = (void *)k_stage<D, FT, 12, true>;
+            k.stage_own[5] = (void *)k_stage<D, FT, 13, true>;
+        }
+    }
     static void fill4(KernelSet &k)
     {
         k.pair2 = (void *)k_pair<D, FT, 2, false>;
-        k.stage4[0] = (void *)k_stage<D, FT, 10>;
-        k.stage4[1] = (void *)k_stage<D, FT, 11>;
-        k.stage4[2] = (void *)k_stage<D, FT, 12>;
-        k.stage4[3] = (void *)k_stage<D, FT, 13>;
         k.rigid4[0] = (void *)k_rigid<D, FT, 10>;
         k.rigid4[1] = (void *)k_rigid<D, FT, 11>;
         k.rigid4[2] = (void *)k_rigid<D, FT, 12>;
@@ -90,15 +101,12 @@ KernelSet kernel_set(int dim, int precision)
 #define GCR_FILL(D_, FT_)                       \
     k.pair0 = StepKernels<D_, FT_>::pair0();    \
     k.pair1 = StepKernels<D_, FT_>::pair1();    \
-    k.stage0 = StepKernels<D_, FT_>::stage0();  \
-    k.stage1 = StepKernels<D_, FT_>::stage1();  \
-    k.stage0f = StepKernels<D_, FT_>::stage0f(); \
-    k.stage1f = StepKernels<D_, FT_>::stage1f(); \
     k.pair_cells[0] = StepKernels<D_, FT_>::pair_cells0(); \
     k.pair_cells[1] = StepKernels<D_, FT_>::pair_cells1(); \
     k.update = StepKernels<D_, FT_>::update();  \
     k.rigid0 = StepKernels<D_, FT_>::rigid0();  \
     k.rigid1 = StepKernels<D_, FT_>::rigid1();  \
+    StepKernels<D_, FT_>::fill_stages(k);        \
     StepKernels<D_, FT_>::fill4(k);
     if (dim == 2 && precision == 0) {
         GCR_FILL(2, double)
