@@ -679,14 +679,11 @@ def run_gpu(args):
         "one_context": dict(one_context, note="the same steps in one context, device-timed; the per-kernel "
                             "profile of `roofline` is of this context") if split else None,
         "e2e": e2e, "roofline": roofline, "clocks": clk,
-        # the run-start check, then 15 kernels per step (two list builds of
-        # four, two pair, two stage, dt rule, update, bookkeeping; 13 when
-        # the stages sum the pair forces; two motor-decision kernels more
-        # with motor populations) in graphs of steps_per_graph steps
         # (per context: each context launches the whole sequence)
-        "gpu_launches": (len(tc.parts) if split else 1) * (1 + ((13 if args.pair_mode == 1 and not groups else 15)
-                                                  + (2 if getattr(specs, "motors", ()) else 0))
-                                             * spg * math.ceil(args.steps / spg)),
+        "gpu_launches": sum(count_launches(args, [specs[i] for i in part], bool(groups),
+                                           bool(getattr(specs, "motors", ())))
+                            for part in (context_parts([sp.n for sp in specs], max(2, args.contexts), groups)
+                                         if split else [range(len(specs))])),
     }
     if fp64 is not None:
         line["fp64"] = fp64
@@ -719,6 +716,26 @@ def split_by_beads(sizes, k):
         cuts.append(min(max(c, cuts[-1] + 1), n - (k - q)))
     cuts.append(n)
     return cuts
+
+
+def count_launches(args, specs, coupled, motors):
+    """Kernel launches of ``args.steps`` steps of one context (csrc/gcr_abi.cu):
+    the run-start check, then one kernel for up to 512 steps while every tile
+    has a CTA of its own (592 of 128 threads; half with coupled populations),
+    else graphs of steps_per_graph steps with, per step, two list builds of two
+    kernels, three of per-system work, two stages and the update, two pair
+    kernels (none where the stages sum the pair forces: 2D mixed precision and
+    pair_mode 1, without coupled populations), two sorts in pair_mode 2 and two
+    motor kernels with motor populations."""
+    steps = args.steps_per_graph * math.ceil(args.steps / args.steps_per_graph)
+    tiles = sum(-(-sp.n // args.block_beads) for sp in specs)
+    limit = 148 * (65536 // (128 * args.block_beads)) // (2 if coupled else 1)
+    if args.ctas_per_sm >= 0 and (coupled or args.pair_mode != 2) and tiles <= max(limit, 8):
+        return 1 + -(-steps // 512)
+    mode = 0 if coupled else args.pair_mode
+    own = not coupled and mode != 2 and (mode == 1 or (specs[0].dim == 2 and args.precision == "mixed"))
+    per_step = 10 + (0 if own else 2) + (2 if mode == 2 else 0) + (2 if motors else 0)
+    return 2 + per_step * steps
 
 
 def context_parts(sizes, k, groups=()):
