@@ -681,7 +681,9 @@ def run_gpu(args):
         "e2e": e2e, "roofline": roofline, "clocks": clk,
         # (per context: each context launches the whole sequence)
         "gpu_launches": sum(count_launches(args, [specs[i] for i in part], bool(groups),
-                                           bool(getattr(specs, "motors", ())))
+                                           bool(getattr(specs, "motors", ())),
+                                           (args.ctas_per_sm or args.split_ctas_per_sm) if split
+                                           else args.ctas_per_sm)
                             for part in (context_parts([sp.n for sp in specs], max(2, args.contexts), groups)
                                          if split else [range(len(specs))])),
     }
@@ -718,11 +720,11 @@ def split_by_beads(sizes, k):
     return cuts
 
 
-def count_launches(args, specs, coupled, motors):
+def count_launches(args, specs, coupled, motors, ctas_per_sm):
     """Kernel launches of ``args.steps`` steps of one context (csrc/gcr_abi.cu):
     the run-start check, then one kernel for up to 512 steps while every tile
-    has a CTA of its own (592 of 128 threads; half with coupled populations),
-    else graphs of steps_per_graph steps with, per step, two list builds of two
+    has a CTA of its own (592 of 128 threads, half with coupled populations, 16
+    in a context of several), else graphs of steps_per_graph steps with, per step, two list builds of two
     kernels, three of per-system work, two stages and the update, two pair
     kernels (none where the stages sum the pair forces: 2D mixed precision and
     pair_mode 1, without coupled populations), two sorts in pair_mode 2 and two
@@ -730,7 +732,8 @@ def count_launches(args, specs, coupled, motors):
     steps = args.steps_per_graph * math.ceil(args.steps / args.steps_per_graph)
     tiles = sum(-(-sp.n // args.block_beads) for sp in specs)
     limit = 148 * (65536 // (128 * args.block_beads)) // (2 if coupled else 1)
-    if args.ctas_per_sm >= 0 and (coupled or args.pair_mode != 2) and tiles <= max(limit, 8):
+    limit = 16 if ctas_per_sm > 0 else max(limit, 8)
+    if ctas_per_sm >= 0 and (coupled or args.pair_mode != 2) and tiles <= limit:
         return 1 + -(-steps // 512)
     mode = 0 if coupled else args.pair_mode
     own = not coupled and mode != 2 and (mode == 1 or (specs[0].dim == 2 and args.precision == "mixed"))

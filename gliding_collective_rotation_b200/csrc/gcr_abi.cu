@@ -806,6 +806,9 @@ bool one_kernel_steps(gcr_ctx *c)
     if (c->cfg.ctas_per_sm < 0 || c->cfg.pair_mode == 2) return false;
     const int kind = steps_kind(c), bb = c->cfg.block_beads;
     const int64_t tiles = (int64_t)c->h_bead_tiles.size();
+    // a context told to leave room for others (ctas_per_sm) launches: cooperative
+    // kernels that do not fit together run one after another
+    if (c->cfg.ctas_per_sm > 0 && tiles > 16) return false;
     // no more than the registers allow fit; a portable cluster always does
     // (the device is asked only where that leaves it open: a query takes longer
     // than a step)
@@ -824,7 +827,6 @@ bool one_kernel_steps(gcr_ctx *c)
     if (tiles <= 16 && c->wide_steps[kind] > 0) return true;
     if (c->grid_steps[kind] == 0) {
         int64_t fit = (int64_t)clusters_that_fit(c, fn, kTeamCluster, bb, c->steps_smem) * kTeamCluster;
-        if (c->cfg.ctas_per_sm > 0) fit = std::min<int64_t>(fit, (int64_t)c->cfg.ctas_per_sm * c->sm_count);
         c->grid_steps[kind] = std::max(1, (int)(fit - fit % kTeamCluster));
     }
     return tiles <= c->grid_steps[kind] / (kind == 0 ? 1 : 2);

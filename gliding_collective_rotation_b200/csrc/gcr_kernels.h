@@ -25,7 +25,7 @@ struct BatchArgs {
     double *xref;  // positions at the last list build, FP64 [bead][dim]
     void *xi;      // translational noise of the current step per bead, FT [bead][dim]
     void *fp;      // pair force per bead (bead order), FT [bead][dim]
-    int *work;     // flagged systems of the coming list build (k_lists_plan)
+    int *work;     // flagged systems of the coming list build (plan_lists)
     int build_cap; // list entries a thread of the build sorts in shared memory
     int n_slots;
     int64_t list_stride;

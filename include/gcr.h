@@ -86,13 +86,14 @@ typedef struct {
     int32_t cell_depth;       /* bead slots per GPU cell: 8, 16, 32, 64 or 128 */
     int32_t block_beads;      /* threads per CTA of bead kernels (64..512) */
     int32_t block_cells;      /* threads per CTA of the cell kernel (64..512) */
-    int32_t steps_per_graph;  /* SRK2 steps per captured CUDA graph (1..64) */
+    int32_t steps_per_graph;  /* steps per captured CUDA graph (1..64); gcr_run takes a multiple of it */
     int32_t ctas_per_sm;      /* persistent CTAs per SM (0 = from occupancy, <0 = one CTA per tile) */
     int32_t list_depth;       /* neighbour-list slots per bead, 4..1024 (0 = 32 in 2D, 96 in 3D) */
     int32_t srk_order;        /* config.SRK_order: 2 (0 = 2) or 4 (SRK.py:144-215, 296-321) */
     int32_t pair_mode;        /* pair forces of SRK2 contexts while no system is coupled to another
                                  population (SRK4 and coupled systems always use 0):
-                                 0: a pair kernel walks each bead's neighbour list;
+                                 0: each bead's neighbour list is walked, by a pair kernel or by the
+                                    stage kernels, whichever is the faster;
                                  1: the stage kernels walk the lists themselves (no pair launch;
                                     the same bits as 0);
                                  2: a cell-staged pair kernel: each CTA copies a row of cells and
