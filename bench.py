@@ -726,8 +726,8 @@ def count_launches(args, specs, coupled, motors, ctas_per_sm):
     has a CTA of its own (592 of 128 threads, half with coupled populations, 16
     in a context of several), else graphs of steps_per_graph steps with, per step, two list builds of two
     kernels, three of per-system work, two stages and the update, two pair
-    kernels (none where the stages sum the pair forces: 2D mixed precision and
-    pair_mode 1, without coupled populations), two sorts in pair_mode 2 and two
+    kernels (none where the stages sum the pair forces: 2D mixed precision in a
+    context alone and pair_mode 1, without coupled populations), two sorts in pair_mode 2 and two
     motor kernels with motor populations."""
     steps = args.steps_per_graph * math.ceil(args.steps / args.steps_per_graph)
     tiles = sum(-(-sp.n // args.block_beads) for sp in specs)
@@ -736,7 +736,7 @@ def count_launches(args, specs, coupled, motors, ctas_per_sm):
     if ctas_per_sm >= 0 and (coupled or args.pair_mode != 2) and tiles <= limit:
         return 1 + -(-steps // 512)
     mode = 0 if coupled else args.pair_mode
-    own = not coupled and mode != 2 and (mode == 1 or (specs[0].dim == 2 and args.precision == "mixed"))
+    own = not coupled and mode != 2 and (mode == 1 or (ctas_per_sm <= 0 and specs[0].dim == 2 and args.precision == "mixed"))
     per_step = 10 + (0 if own else 2) + (2 if mode == 2 else 0) + (2 if motors else 0)
     return 2 + per_step * steps
 
@@ -1091,7 +1091,7 @@ def main():
     ap.add_argument("--plain", type=int, default=1)
     ap.add_argument("--plain-steps", type=int, default=50)
     ap.add_argument("--e2e-steps-per-call", type=int, default=100)
-    ap.add_argument("--split-ctas-per-sm", type=int, default=6,
+    ap.add_argument("--split-ctas-per-sm", type=int, default=9,
                     help="persistent CTAs per SM of each context when the systems are split over several "
                          "(0: as many as fit); --ctas-per-sm, when given, sets both")
     ap.add_argument("--contexts", type=int, default=4, choices=range(1, 9),

@@ -662,14 +662,18 @@ int enqueue_step4(gcr_ctx *c)
 int pair_mode(const gcr_ctx *c, bool cross) { return (c->cfg.srk_order == 2 && !cross) ? c->cfg.pair_mode : 0; }
 
 // The stages walk the lists themselves (pair_mode 1, the same bits as 0) in 2D
-// mixed precision whatever the mode: the sweep's step takes 645 us so, 678 with
-// the pair kernel, 16 SRK4 systems 145 against 155.  Elsewhere only when asked for: in FP64 the 64-system
-// sweep's two stages take 233 us so, 224 with the pair kernel (registers), and
-// 3D lists are long (505 against 377 us).
+// mixed precision: the sweep's step takes 645 us so, 678 with the pair kernel,
+// 16 SRK4 systems 145 against 155.  Elsewhere only when asked for: in FP64 the
+// 64-system sweep's two stages take 233 us so, 224 with the pair kernel
+// (registers), and 3D lists are long (505 against 377 us).  Nor in a context
+// that shares the device (ctas_per_sm > 0): its neighbours fill the ends of the
+// shorter kernels, and the pair kernel holds fewer registers; the sweep over
+// four contexts runs 8.37e9 bead-steps/s with it against 7.96e9 at 6 CTAs per
+// SM, 8.50e9 against 8.43e9 at 9.
 bool own_pair(const gcr_ctx *c, bool cross)
 {
     if (cross) return false;
-    if (c->cfg.dim == 2 && c->cfg.precision == GCR_MIXED) return pair_mode(c, cross) != 2;
+    if (c->cfg.dim == 2 && c->cfg.precision == GCR_MIXED && c->cfg.ctas_per_sm <= 0) return pair_mode(c, cross) != 2;
     return pair_mode(c, cross) == 1;
 }
 
