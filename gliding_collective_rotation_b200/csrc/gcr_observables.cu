@@ -101,12 +101,16 @@ __device__ __forceinline__ long long pair_bin(double d2, double binsize, float i
 // launches.  One pair a thread, with its row found by a square root, a sine
 // and a cosine of both angles for every pair and three allocations a call took
 // 185 us a call for g(r) and 265 us for Cvv and Cnn of 4000 chains; so 85 and
-// 102 us (B200, host to host; the kernel 38 and 52 us).
-constexpr int kPairTile = 64, kPairGroups = 4;
+// 102 us (B200, host to host; the kernel 38 and 52 us).  While there are fewer
+// tiles than groups on the SMs, a tile's columns are cut into up to kPairSlices
+// slices, a group each: a thread that walks all 64 alone is the time of a call
+// with few chains (the five calls of an analysis of 50, 500 and 1400 chains 355,
+// 392 and 397 us with whole tiles, 288, 307 and 353 so).
+constexpr int kPairTile = 64, kPairGroups = 4, kPairSlices = 16;
 
 __global__ void __launch_bounds__(kPairTile *kPairGroups)
     k_pair_corr(const double *__restrict__ com, const double *__restrict__ trig, int n_chains, double L, double binsize,
-                int n_bins, int kind, unsigned long long *counts, unsigned long long *sums)
+                int n_bins, int kind, int slices, unsigned long long *counts, unsigned long long *sums)
 {
     extern __shared__ unsigned long long sh_hist[];  // kinds 1, 2: [n_bins] fixed-point sums; [n_bins] 32-bit counts
     unsigned long long *hs = sh_hist;
@@ -120,9 +124,11 @@ __global__ void __launch_bounds__(kPairTile *kPairGroups)
     const double *cx = col[group][0], *cy = col[group][1], *tc = col[group][2], *ts = col[group][3];
     const float inv = (float)(1.0 / binsize);
     const int tiles = (n_chains + kPairTile - 1) / kPairTile;
-    const long long n_tiles = (long long)tiles * (tiles + 1) / 2;
+    const long long n_tiles = (long long)tiles * (tiles + 1) / 2 * slices;
+    const int width = kPairTile / slices;
     for (long long t0 = (long long)blockIdx.x * kPairGroups; t0 < n_tiles; t0 += (long long)gridDim.x * kPairGroups) {
-        const long long t = t0 + group;
+        const long long item = t0 + group, t = item / slices;
+        const int k0 = (int)(item % slices) * width;  // the first of this slice's columns
         // tile t of the lower triangle -> (I, J), J <= I
         long long I = (long long)((sqrt(1.0 + 8.0 * (double)t) - 1.0) * 0.5);
         while (I * (I + 1) / 2 > t) I--;
@@ -130,7 +136,7 @@ __global__ void __launch_bounds__(kPairTile *kPairGroups)
         const long long J = t - I * (I + 1) / 2;
         const long long i = I * kPairTile + lane, j0 = J * kPairTile;
         __syncthreads();  // the previous columns are done with
-        if (t < n_tiles && j0 + lane < n_chains) {
+        if (item < n_tiles && j0 + lane < n_chains) {
             const size_t j = (size_t)(j0 + lane) * 2;
             col[group][0][lane] = com[j];
             col[group][1][lane] = com[j + 1];
@@ -140,11 +146,12 @@ __global__ void __launch_bounds__(kPairTile *kPairGroups)
             }
         }
         __syncthreads();
-        if (t >= n_tiles || i >= n_chains) continue;
+        if (item >= n_tiles || i >= n_chains) continue;
         const double x = com[(size_t)i * 2], y = com[(size_t)i * 2 + 1];
         const double ca = kind != 0 ? trig[(size_t)i * 2] : 0.0, sa = kind != 0 ? trig[(size_t)i * 2 + 1] : 0.0;
         const int cols = (int)min((long long)kPairTile, i - j0);  // the columns below the diagonal
-        for (int k = 0; k < cols; k++) {
+        const int k1 = min(cols, k0 + width);
+        for (int k = k0; k < k1; k++) {
             const double s0 = centre_sep(x, cx[k], L), s1 = centre_sep(y, cy[k], L);
             const long long bin = pair_bin(__dadd_rn(__dmul_rn(s0, s0), __dmul_rn(s1, s1)), binsize, inv);
             if (bin < 0 || bin >= n_bins) continue;  // past the last bin of the reference's range
@@ -196,13 +203,17 @@ cudaError_t launch_pair_corr(const double *com, const double *trig, int n_chains
         if (e != cudaSuccess) return e;
     }
     const long long tiles = (n_chains + kPairTile - 1) / kPairTile;
-    const long long n_tiles = tiles * (tiles + 1) / 2, groups = (n_tiles + kPairGroups - 1) / kPairGroups;
+    // no more slices than fill one CTA on each SM
+    int slices = 1;
+    while (slices < kPairSlices && tiles * (tiles + 1) / 2 * (2 * slices) <= (long long)kPairGroups * sm_count)
+        slices *= 2;
+    const long long n_tiles = tiles * (tiles + 1) / 2 * slices, groups = (n_tiles + kPairGroups - 1) / kPairGroups;
     // few CTAs, as each adds its histogram to the result; enough that a CTA's
-    // 32-bit counts hold its pairs (2 * kPairTile^2 a tile: 2^18 tiles)
+    // 32-bit counts hold its pairs (2 * kPairTile^2 a whole tile: 2^18 of them)
     long long blocks = groups > 4LL * sm_count ? 4LL * sm_count : groups;
     blocks = blocks > n_tiles / 262144 + 1 ? blocks : n_tiles / 262144 + 1;
     k_pair_corr<<<(unsigned)blocks, kPairTile * kPairGroups, smem, st>>>(com, trig, n_chains, L, binsize, n_bins, kind,
-                                                                         counts, sums);
+                                                                         slices, counts, sums);
     return cudaGetLastError();
 }
 
