@@ -105,7 +105,7 @@ __device__ __forceinline__ long long pair_bin(double d2, double binsize, float i
 // tiles than groups on the SMs, a tile's columns are cut into up to kPairSlices
 // slices, a group each: a thread that walks all 64 alone is the time of a call
 // with few chains (the five calls of an analysis of 50, 500 and 1400 chains 355,
-// 392 and 397 us with whole tiles, 288, 307 and 353 so).
+// 392 and 397 us with whole tiles, 288, 307 and 348 so).
 constexpr int kPairTile = 64, kPairGroups = 4, kPairSlices = 16;
 
 __global__ void __launch_bounds__(kPairTile *kPairGroups)
@@ -203,9 +203,10 @@ cudaError_t launch_pair_corr(const double *com, const double *trig, int n_chains
         if (e != cudaSuccess) return e;
     }
     const long long tiles = (n_chains + kPairTile - 1) / kPairTile;
-    // no more slices than fill one CTA on each SM
+    // no more slices than fill two CTAs on each SM: 1400 and 1500 chains 348 and
+    // 458 us, 364 and 497 at one, the same at four
     int slices = 1;
-    while (slices < kPairSlices && tiles * (tiles + 1) / 2 * (2 * slices) <= (long long)kPairGroups * sm_count)
+    while (slices < kPairSlices && tiles * (tiles + 1) / 2 * slices <= (long long)kPairGroups * sm_count)
         slices *= 2;
     const long long n_tiles = tiles * (tiles + 1) / 2 * slices, groups = (n_tiles + kPairGroups - 1) / kPairGroups;
     // few CTAs, as each adds its histogram to the result; enough that a CTA's

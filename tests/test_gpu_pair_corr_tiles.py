@@ -21,7 +21,7 @@ from gliding_collective_rotation_b200.workloads import SystemSpec  # noqa: E402
 from oracle import observables as OB  # noqa: E402
 
 
-@pytest.mark.parametrize("n", [2, 63, 64, 65, 128, 129, 257, 700, 1000, 1400, 1500])
+@pytest.mark.parametrize("n", [2, 63, 64, 65, 128, 129, 257, 700, 1000, 1400, 1500, 2300])
 @pytest.mark.parametrize("lattice,binsize", [(False, 0.25), (True, 0.25), (False, 0.1), (True, 0.1)])
 def test_pair_correlation_at_tile_and_bin_edges(n, lattice, binsize):
     rs = np.random.default_rng([n, lattice])
