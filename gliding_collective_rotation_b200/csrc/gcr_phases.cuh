@@ -2479,6 +2479,9 @@ __global__ void __maxnreg__(128)
 {
     Team team{ts, 0, 0, csize};
     const Span sp = bead_span(A);
+    // the CTAs of a cluster are scheduled together but start one by one: a
+    // CTA's shared memory may be written by another only once it runs
+    cluster_sync();
     unsigned info = team.sync(A, kDutyStart);
     bool raised = false;
     for (int k = 0; k < steps; k++) {
