@@ -1002,7 +1002,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     e = e ? e : cudaMalloc(&c->xref, sizeof(double) * (size_t)cfg.bead_capacity * cfg.dim);
     e = e ? e : cudaMalloc(&c->img, sizeof(int) * (size_t)cfg.bead_capacity * cfg.dim);
     e = e ? e : cudaMalloc(&c->restb, sizeof(double) * (size_t)cfg.bead_capacity);
-    e = e ? e : cudaMalloc(&c->work, sizeof(int) * (size_t)(3 + 3 * (S + 1)));
+    e = e ? e : cudaMalloc(&c->work, sizeof(int) * (size_t)(3 * S + 6));
     e = e ? e : cudaMalloc(&c->team, sizeof(TeamSync));
     e = e ? e : cudaMalloc(&c->xi, (size_t)cfg.bead_capacity * cfg.dim * (cfg.precision == GCR_FP64 ? 8 : 4));
     e = e ? e : cudaMalloc(&c->fp, (size_t)cfg.bead_capacity * cfg.dim * (cfg.precision == GCR_FP64 ? 8 : 4));
@@ -1021,7 +1021,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     for (int *cnt : c->cnt) cudaMemsetAsync(cnt, 0, sizeof(int) * cells_alloc, c->stream);
     cudaMemsetAsync(c->ncount, 0, sizeof(int) * (size_t)cfg.bead_capacity, c->stream);
     cudaMemsetAsync(c->img, 0, sizeof(int) * (size_t)cfg.bead_capacity * cfg.dim, c->stream);
-    cudaMemsetAsync(c->work, 0, sizeof(int) * (size_t)(3 + 3 * (S + 1)), c->stream);
+    cudaMemsetAsync(c->work, 0, sizeof(int) * (size_t)(3 * S + 6), c->stream);
     c->slots.assign(S, Slot());
     c->hP.assign(S, SysP());
     c->hS.assign(S, SysS());

@@ -279,13 +279,15 @@ __device__ __forceinline__ Span bead_span(const BatchArgs &A)
 // Work list of a list build: the flagged systems, compacted, with the
 // running sum of their bead tiles and cell tiles.  Layout of A.work:
 //   [0] flagged systems m, [1] their bead tiles, [2] their cell tiles,
-//   then sys[S], bead_prefix[S+1], cell_prefix[S+1] (S = slot count).
+//   then sys[S], bead_prefix[S+1], cell_prefix[S+1] (S = slot count) and a
+//   word that the binning sets when it finds a bead outside its box.
 // Built by one CTA (step_duty) before each stage's list kernels, which then
 // visit the tiles of flagged systems only, and leave at once when there are
 // none.
 struct Work {
     int m, n_bead, n_cell;
     const int *sys, *bead0, *cell0;
+    int *outside;
 };
 
 __device__ __forceinline__ Work work_list(const BatchArgs &A)
@@ -298,6 +300,7 @@ __device__ __forceinline__ Work work_list(const BatchArgs &A)
     w.sys = q + 3;
     w.bead0 = w.sys + A.n_slots;
     w.cell0 = w.bead0 + A.n_slots + 1;
+    w.outside = A.work + (w.cell0 + A.n_slots + 1 - q);
     return w;
 }
 
@@ -401,6 +404,7 @@ static __device__ __noinline__ int plan_lists(const BatchArgs &A)
         q[0] = carry[0];
         q[1] = carry[1];
         q[2] = carry[2];
+        wc[A.n_slots + 1] = 0;
         wb[carry[0]] = carry[1];
         wc[carry[0]] = carry[2];
     }
@@ -556,6 +560,9 @@ __device__ __forceinline__ void bin_tiles(const BatchArgs &A, Span sp)
         for (int i = 0; i < D; i++) x[i] = X[(size_t)b * D + i];
         int ci[3];
         cell_of<D>(p, x, ci);
+#pragma unroll
+        for (int i = 0; i < D; i++)
+            if (!(x[i] >= 0.0 && x[i] <= p.L)) *w.outside = 1;
         const int64_t gc = p.cell_off + ((int64_t)ci[2] * p.nc + ci[1]) * p.nc + ci[0];
         const int slot = atomicAdd(cell_counts(A, s.turn) + gc, 1);
         if (slot < A.depth)
@@ -682,10 +689,13 @@ struct ListInsert {
 // separation is a plain difference, as the periodic shift between a bead and a
 // neighbour cell is the cell's (a pair within the list radius meets through no
 // other image: the grid has 3 cells a side or more, each at least that wide),
-// and its rounding is far inside the margin of the list radius.
-template <int D, typename Take>
+// and its rounding is far inside the margin of the list radius.  LOOSE: x is the
+// bead's own position and the separation the minimum image.  A build takes that
+// form while the caller's positions leave the box (a step wraps them): a bead
+// outside is in a cell at the edge, wherever its images are.
+template <int D, bool LOOSE, typename Take>
 __device__ __forceinline__ void scan_cell(const double *X, int n, const double *x, const int *it, int m, double rl2,
-                                          bool &bad, Take take)
+                                          double L, bool &bad, Take take)
 {
     int j_next = m > 0 ? it[0] : 0;
     for (int q = 0; q < m; q++) {
@@ -698,7 +708,8 @@ __device__ __forceinline__ void scan_cell(const double *X, int n, const double *
         double ds = 0.0;
 #pragma unroll
         for (int i = 0; i < D; i++) {
-            const double d = X[(size_t)j * D + i] - x[i];
+            const double xj = X[(size_t)j * D + i];
+            const double d = LOOSE ? inbounds(xj, x[i], 0.5 * L, L) : xj - x[i];
             ds += d * d;
         }
         if (ds <= rl2) take(j);
@@ -791,22 +802,11 @@ __device__ void build_cross(const BatchArgs &A, const SysP &p, SysS &s, int c, i
 // its beads' cells).  First builds, B200, with the per-cell sort that lists
 // sorted as they are built do not need: 64 sweep systems 215 -> 147 us, 300k
 // 3D beads 442 -> 395 us, 48 boxes of two populations 272 -> 214 us.
-// The cells of the flagged systems have their other counts zeroed for the
-// next binning.
-template <int D, int WHICH>
-__device__ __forceinline__ void build_tiles(const BatchArgs &A, Span sp)
+template <int D, int WHICH, bool LOOSE>
+__device__ __forceinline__ void build_lists(const BatchArgs &A, const Work &w, Span sp)
 {
     extern __shared__ __align__(16) unsigned char build_smem[];
     int *col = reinterpret_cast<int *>(build_smem) + threadIdx.x;
-    const Work w = work_list(A);
-    for (int t = sp.first; t < w.n_cell; t += sp.step) {
-        const int k = work_owner(w.cell0, w.m, t);
-        const int sys = w.sys[k];
-        const SysP &p = A.P[sys];
-        int *other = cell_counts(A, A.S[sys].turn + 1);
-        const int c0 = (t - w.cell0[k]) * A.tile_cells, c1 = min(c0 + A.tile_cells, p.n_cells);
-        for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) other[p.cell_off + c] = 0;
-    }
     for (int t = sp.first; t < w.n_bead; t += sp.step) {
         const int k = work_owner(w.bead0, w.m, t);
         const int sys = w.sys[k];
@@ -856,9 +856,11 @@ __device__ __forceinline__ void build_tiles(const BatchArgs &A, Span sp)
                 for (int dx = 0; dx < 3; dx++) {
                     const int mm = m[dx] < 0 ? 0 : (m[dx] < A.depth ? m[dx] : A.depth);
                     xs[0] = x0[dx];
-                    scan_cell<D>(X, n, xs, A.items + ((row + cx[dx]) << A.log_depth), mm, p.rl2, bad, [&](int j) {
-                        if (j < ex_lo || j > ex_hi) list.add(j);  // b itself is in the excluded range
-                    });
+                    scan_cell<D, LOOSE>(X, n, LOOSE ? x : xs, A.items + ((row + cx[dx]) << A.log_depth), mm, p.rl2,
+                                        p.L, bad, [&](int j) {
+                                            // b itself is in the excluded range
+                                            if (j < ex_lo || j > ex_hi) list.add(j);
+                                        });
                 }
             }
         }
@@ -870,6 +872,33 @@ __device__ __forceinline__ void build_tiles(const BatchArgs &A, Span sp)
         if (bad) atomicOr(&s.flags, kFlagListCorrupt);
         for (int c = 0; c < p.n_cross && c < kMaxPops - 1; c++) build_cross<D, WHICH>(A, p, s, c, b, x, col);
     }
+}
+
+// ... out of line, or the form that every step takes would spill
+template <int D, int WHICH>
+static __device__ __noinline__ void build_lists_loose(const BatchArgs &A, Span sp)
+{
+    build_lists<D, WHICH, true>(A, work_list(A), sp);
+}
+
+// the lists of the flagged systems; their cells have the other counts zeroed
+// for the next binning
+template <int D, int WHICH>
+__device__ __forceinline__ void build_tiles(const BatchArgs &A, Span sp)
+{
+    const Work w = work_list(A);
+    for (int t = sp.first; t < w.n_cell; t += sp.step) {
+        const int k = work_owner(w.cell0, w.m, t);
+        const int sys = w.sys[k];
+        const SysP &p = A.P[sys];
+        int *other = cell_counts(A, A.S[sys].turn + 1);
+        const int c0 = (t - w.cell0[k]) * A.tile_cells, c1 = min(c0 + A.tile_cells, p.n_cells);
+        for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) other[p.cell_off + c] = 0;
+    }
+    if (w.n_bead > 0 && *w.outside)
+        build_lists_loose<D, WHICH>(A, sp);
+    else
+        build_lists<D, WHICH, false>(A, w, sp);
 }
 
 template <int D, int WHICH>
