@@ -195,6 +195,13 @@ int build_cap(int block, int list_depth) { return std::min(list_depth <= 32 ? 12
 // ... and in the one-kernel steps, where the CTAs of all tiles share the SMs
 constexpr int kTeamBuildCap = 24;
 
+// their dynamic shared memory: the list walk's buffers or the build's columns
+constexpr int kMaxBlock = 512;
+size_t steps_smem(const gcr_ctx *c, int block, int cap)
+{
+    return std::max(c->ks.pair_smem(block), sizeof(int) * (size_t)cap * block);
+}
+
 // CTAs of a cluster of the one-kernel steps beyond one cluster
 constexpr int kTeamCluster = 8;
 
@@ -209,6 +216,17 @@ int kernel_grid(const gcr_ctx *c, void *fn, int block, int64_t max_tiles, size_t
     int64_t g = (int64_t)c->sm_count * occ;
     g = std::min<int64_t>(g, std::max<int64_t>(max_tiles, 1));
     return (int)std::max<int64_t>(g, 1);
+}
+
+// Dynamic shared memory up to `bytes` for a kernel's launches.  The limit belongs
+// to the kernel, for every context and thread of the process: each caller sets
+// the most that any of them may need, never its own share, so none lowers
+// another's.
+bool allow_smem(void *fn, size_t bytes)
+{
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
 }
 
 // clusters of n CTAs of a kernel that fit the device at once (0: none)
@@ -819,7 +837,7 @@ bool one_kernel_steps(gcr_ctx *c)
     if (tiles > (int64_t)c->sm_count * std::max(1, 65536 / (128 * bb))) return false;
     void *fn = c->ks.steps[kind];
     if (c->grid_steps[kind] < 0) {
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->steps_smem);
+        if (!allow_smem(fn, steps_smem(c, kMaxBlock, kTeamBuildCap))) return false;
         c->grid_steps[kind] = 0;
     }
     if (tiles <= kTeamCluster) return true;
@@ -1048,10 +1066,6 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     a.img = c->img;
     a.restb = c->restb;
     a.row_prefix = c->d_row_prefix;
-    // staging capacity of the cell-staged pair kernel: twice the beads of a
-    // row tile and its neighbour rows at the mean occupancy (the row tiling
-    // aims at block_beads beads per row); a denser tile reads global memory
-    a.cell_stage_cap = 2 * c->ks.pair_cells_rows * cfg.block_beads;
     a.xi = c->xi;
     a.fp = c->fp;
     a.work = c->work;
@@ -1065,35 +1079,42 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     a.order = cfg.srk_order;
     a.mixed = cfg.precision == GCR_MIXED ? 1 : 0;
     c->pair_smem = c->ks.pair_smem(cfg.block_beads);
-    if (c->pair_smem > 48 * 1024)
-        for (void *fn : {c->ks.pair0, c->ks.pair1, c->ks.pair2, c->ks.pair_cross[0], c->ks.pair_cross[1],
-                         c->ks.pair_cross[2]})
-            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->pair_smem);
     for (int k = 0; k < 6; k++) {
         c->grid_stage[k] = kernel_grid(c, c->ks.stage[k], cfg.block_beads, c->max_bead_tiles);
         void *fn = c->ks.stage_own[k];
         if (!fn) continue;
-        if (c->pair_smem > 48 * 1024)
-            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->pair_smem);
         c->grid_stage_own[k] = kernel_grid(c, fn, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
     }
-    c->pair_cells_smem = c->ks.pair_cells_smem(a.cell_stage_cap);
-    if (c->pair_cells_smem > 48 * 1024)
-        for (int k = 0; k < 2; k++)
-            cudaFuncSetAttribute(c->ks.pair_cells[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)c->pair_cells_smem);
-    // row tiles: at most cells/3 rows, plus cells/T <= 2 beads/block_beads (or cells/128) segments
-    c->grid_pair_cells = kernel_grid(c, c->ks.pair_cells[0], cfg.block_beads,
-                                     cfg.cell_capacity / 3 + cfg.cell_capacity / 128 +
-                                         2 * cfg.bead_capacity / cfg.block_beads + S,
-                                     c->pair_cells_smem);
+    if (cfg.pair_mode == 2) {
+        // staging capacity of the cell-staged pair kernel: twice the beads of a
+        // row tile and its neighbour rows at the mean occupancy (the row tiling
+        // aims at block_beads beads per row), as far as shared memory goes; a
+        // denser tile reads global memory
+        cudaFuncAttributes fa = {};
+        int optin = 0;
+        if (cudaFuncGetAttributes(&fa, c->ks.pair_cells[0]) != cudaSuccess ||
+            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess)
+            return cleanup(fail(GCR_ERR_CUDA, "shared memory of the cell-staged pair kernel"));
+        const size_t limit = (size_t)optin - fa.sharedSizeBytes;
+        a.cell_stage_cap = (int)std::min<size_t>(2 * (size_t)c->ks.pair_cells_rows * cfg.block_beads,
+                                                 limit / c->ks.pair_cells_smem(1));
+        c->pair_cells_smem = c->ks.pair_cells_smem(a.cell_stage_cap);
+        for (void *fn : c->ks.pair_cells)
+            if (!allow_smem(fn, limit))
+                return cleanup(fail(GCR_ERR_CUDA, "shared memory of the cell-staged pair kernel"));
+        // row tiles: at most cells/3 rows, plus cells/T <= 2 beads/block_beads (or cells/128) segments
+        c->grid_pair_cells = kernel_grid(c, c->ks.pair_cells[0], cfg.block_beads,
+                                         cfg.cell_capacity / 3 + cfg.cell_capacity / 128 +
+                                             2 * cfg.bead_capacity / cfg.block_beads + S,
+                                         c->pair_cells_smem);
+    }
     c->grid_update = kernel_grid(c, c->ks.update, cfg.block_beads, c->max_bead_tiles);
     c->grid_pair = kernel_grid(c, c->ks.pair0, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
     c->grid_bin = kernel_grid(c, c->ks.bin0, cfg.block_beads, c->max_bead_tiles);
     c->grid_sort = kernel_grid(c, c->ks.sort, cfg.block_cells, c->max_cell_tiles);
     c->grid_build = kernel_grid(c, c->ks.build0, cfg.block_beads, c->max_bead_tiles, c->build_smem);
     c->grid_sys = (int)((S + 127) / 128);
-    c->steps_smem = std::max(c->pair_smem, sizeof(int) * (size_t)std::min(kTeamBuildCap, a.build_cap) * cfg.block_beads);
+    c->steps_smem = steps_smem(c, cfg.block_beads, std::min(kTeamBuildCap, a.build_cap));
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return cleanup(fail(GCR_ERR_CUDA, "initialisation"));
     *out = c;
     return GCR_OK;
@@ -1799,7 +1820,7 @@ int gcr_pair_correlation(gcr_ctx *c, int32_t slot, int32_t kind, double binsize,
     // bins of np.arange(0, int(L/2) * sqrt(2), binsize)
     const double stop = (double)(int64_t)(p.L / 2.0) * std::sqrt(2.0);
     const int64_t n_bins = (int64_t)std::ceil(stop / binsize);
-    if (n_bins < 1 || n_bins > 12000) return fail(GCR_ERR_BAD_ARG, "binsize gives more than 12000 bins");
+    if (n_bins < 1 || n_bins > kMaxCorrBins) return fail(GCR_ERR_BAD_ARG, "binsize gives more than 12000 bins");
     const int nc = p.n_chains;
     if (kind != 0 && (int64_t)nc * (nc - 1) > ((int64_t)1 << 31))
         return fail(GCR_ERR_BAD_ARG, "Cvv / Cnn are limited to about 46000 chains (fixed-point sums)");

@@ -138,6 +138,7 @@ cudaError_t launch_export_list(const int *nbr, const int *ncount, int64_t stride
 // com, phi, trig may be null; trig: cosine and sine of the chains' angle of 1- or 2-fold symmetry (sym)
 cudaError_t launch_chain_frames(int dim, int precision, const SysP &p, const int32_t *chain_start, double *com,
                                 double *phi, int sym, double *trig, cudaStream_t st);
+constexpr int kMaxCorrBins = 12000;
 cudaError_t launch_pair_corr(const double *com, const double *trig, int n_chains, double L, double binsize, int n_bins,
                              int kind, unsigned long long *counts, unsigned long long *sums, int sm_count,
                              cudaStream_t st);

@@ -199,7 +199,9 @@ cudaError_t launch_pair_corr(const double *com, const double *trig, int n_chains
 {
     const size_t smem = (size_t)n_bins * ((kind != 0 ? sizeof(unsigned long long) : 0) + sizeof(unsigned));
     if (smem > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_pair_corr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the limit is every caller's: always that of the largest histogram
+        const int limit = kMaxCorrBins * (int)(sizeof(unsigned long long) + sizeof(unsigned));
+        cudaError_t e = cudaFuncSetAttribute(k_pair_corr, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
         if (e != cudaSuccess) return e;
     }
     const long long tiles = (n_chains + kPairTile - 1) / kPairTile;

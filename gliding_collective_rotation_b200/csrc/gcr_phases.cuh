@@ -1056,6 +1056,8 @@ constexpr int team_row_ahead()
 template <int D, typename FT>
 size_t pair_smem_bytes(int TB)
 {
+    // what a launch may take without asking, at the widest block
+    static_assert((512 / 32) * 4 * 32 * kPairChunk * sizeof(double) <= 48 * 1024, "dynamic shared memory");
     return (size_t)(TB / 32) * (D + 1) * 32 * kPairChunk * sizeof(FT);
 }
 
