@@ -20,6 +20,7 @@ ERRORS = {-1: "BAD_ARG", -2: "CUDA", -3: "OOM", -4: "NONFINITE", -5: "TIMEOUT", 
 GCR_FP64, GCR_MIXED = 0, 1
 FLAG_CELL_OVERFLOW, FLAG_NONFINITE, FLAG_NEXT_OVERFLOW, FLAG_LIST_CORRUPT, FLAG_LIST_OVERFLOW = 1, 2, 4, 8, 16
 FLAG_SERIES_FULL = 32
+FLAG_WAIT_EXPIRED = 64
 
 
 class GcrError(RuntimeError):

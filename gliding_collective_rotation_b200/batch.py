@@ -18,7 +18,7 @@ import math
 import numpy as np
 import torch
 
-from ._lib import FLAG_CELL_OVERFLOW, FLAG_LIST_OVERFLOW, FLAG_NEXT_OVERFLOW
+from ._lib import FLAG_CELL_OVERFLOW, FLAG_LIST_OVERFLOW, FLAG_NEXT_OVERFLOW, FLAG_WAIT_EXPIRED
 from .engine import Engine, SystemState, default_config, default_skin, footprint
 
 OVERFLOW = FLAG_CELL_OVERFLOW | FLAG_NEXT_OVERFLOW | FLAG_LIST_OVERFLOW
@@ -185,6 +185,8 @@ class Batch:
         over, so the noise stream goes on."""
         sts = self.statuses()
         flags = 0
+        if any(s["flags"] & FLAG_WAIT_EXPIRED for s in sts):
+            raise RuntimeError("a system stopped in the middle of a step: its state cannot be carried on")
         for st, s in zip(self.states, sts):
             st.params.step = s["step"]
             flags |= s["flags"]

@@ -166,6 +166,7 @@ struct gcr_ctx {
     int grid_stage[6] = {}, grid_stage_own[6] = {};
     int grid_pair_cells = 1;
     TeamSync *team = nullptr;          // barrier state of the one-kernel steps
+    int team_polls = 1 << 23;          // of a waiting CTA before it gives up: some hundred ns each, the longest phase a few ms
     int grid_steps[3] = {-1, -1, -1};  // CTAs of them that fit at once, in clusters of kTeamCluster (-1: not asked)
     int wide_steps[3] = {-1, -1, -1};  // a cluster of 16 CTAs fits
     std::vector<int64_t> attempts;     // steps queued per slot since it was armed
@@ -868,7 +869,7 @@ int launch_steps(gcr_ctx *c, int64_t steps)
     GCR_CUDA(cudaMemsetAsync(c->team, 0, sizeof(TeamSync), c->stream));
     BatchArgs args = c->args;
     args.build_cap = std::min(kTeamBuildCap, args.build_cap);
-    void *a[] = {&args, &c->team, &n, &csize, &motor, &rigid};
+    void *a[] = {&args, &c->team, &n, &csize, &motor, &rigid, &c->team_polls};
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(grid);
     lc.blockDim = dim3(c->cfg.block_beads);
@@ -998,6 +999,8 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     {
         const char *e = std::getenv("GCR_PDL");
         c->pdl = !(e && e[0] == '0');
+        e = std::getenv("GCR_TEAM_POLLS");
+        if (e && std::atoi(e) > 0) c->team_polls = std::atoi(e);
     }
     const int64_t S = cfg.system_capacity;
     c->max_bead_tiles = cfg.bead_capacity / cfg.block_beads + S;
@@ -1492,6 +1495,13 @@ int check_call(const gcr_call *call)
     return GCR_OK;
 }
 
+// a system that the one-kernel steps gave up on is a step apart in its parts
+int check_whole(const SysS &s)
+{
+    if (!(s.flags & kFlagWaitExpired)) return GCR_OK;
+    return fail(GCR_ERR_STATE, "the system stopped in the middle of a step: evict it and admit a state that is whole");
+}
+
 // arm one system for a call; true when its last call ended in a stop (a
 // fatal flag), after which its lists are rebuilt from zeroed cell counts
 bool arm(SysS &s, const gcr_call *call)
@@ -1533,6 +1543,8 @@ int gcr_call_begin_batch(gcr_ctx *c, int32_t n, const int32_t *slots, const gcr_
     // the device table holds the step counters: fetch it, arm, write it back
     GCR_CUDA(cudaMemcpyAsync(c->hS.data(), c->dS, sizeof(SysS) * S, cudaMemcpyDeviceToHost, c->stream));
     GCR_CUDA(cudaStreamSynchronize(c->stream));
+    for (int i = 0; i < n; i++)
+        if (int rc = check_whole(c->hS[slots[i]])) return rc;
     std::vector<int> stopped;
     for (int i = 0; i < n; i++) {
         if (arm(c->hS[slots[i]], calls + i)) stopped.push_back(slots[i]);
@@ -1556,6 +1568,7 @@ int gcr_call_begin(gcr_ctx *c, int32_t slot, const gcr_call *call)
     // the device copy holds the current step counter: fetch it first
     GCR_CUDA(cudaMemcpyAsync(&s, c->dS + slot, sizeof(SysS), cudaMemcpyDeviceToHost, c->stream));
     GCR_CUDA(cudaStreamSynchronize(c->stream));
+    if ((rc = check_whole(s))) return rc;
     const bool stopped = arm(s, call);
     c->attempts[slot] = 0;
     GCR_CUDA(cudaMemcpyAsync(c->dS + slot, &s, sizeof(SysS), cudaMemcpyHostToDevice, c->stream));

@@ -45,8 +45,10 @@ constexpr int kFlagNextOverflow = 4;
 constexpr int kFlagListCorrupt = 8;  // an inconsistent cell or neighbour list was detected and not used
 constexpr int kFlagListOverflow = 16;  // more list partners of a bead than the list depth
 constexpr int kFlagSeriesFull = 32;    // the series buffer was full (not fatal)
+constexpr int kFlagWaitExpired = 64;   // the one-kernel steps gave up: parts of the system are a step apart
 // a system with one of these stops: every kernel skips it until re-armed
-constexpr int kFlagFatal = kFlagCellOverflow | kFlagNonFinite | kFlagListCorrupt | kFlagListOverflow;
+constexpr int kFlagFatal =
+    kFlagCellOverflow | kFlagNonFinite | kFlagListCorrupt | kFlagListOverflow | kFlagWaitExpired;
 
 struct SysP {
     // caller-owned state

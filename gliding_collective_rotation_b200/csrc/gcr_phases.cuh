@@ -2348,15 +2348,13 @@ __global__ void __launch_bounds__(512) k_motor(const __grid_constant__ BatchArgs
 // A team of up to 16 CTAs is one thread-block cluster and meets at its
 // hardware barrier.  A larger one is a cooperative launch of clusters that
 // meet at a counter in global memory; every wait there is bounded: a CTA
-// that gives up stops every system (kFlagListCorrupt) and the team returns.
+// that gives up stops every running system (kFlagWaitExpired) and the team
+// returns.  It may have left its beads a step behind the others', so such a
+// system can only be admitted again.
 // KIND: 0 SRK2 of uncoupled systems without the rigid-rod projection (the
 // stage sums its pair forces itself); 1 every SRK2 batch; 2 every SRK4 batch.
 // ------------------------------------------------------------------------
 constexpr unsigned kTeamLists = 1, kTeamStop = 2;
-// polls before a waiting CTA gives up: each takes some hundred ns, the longest
-// phase a few ms
-constexpr int kTeamPolls = 1 << 23;
-
 // one CTA: a duty between two phases; ask: some thread asked for a list build
 // since the last plan
 static __device__ __noinline__ unsigned team_duty(const BatchArgs &A, int duty, bool ask)
@@ -2397,6 +2395,7 @@ struct Team {
     unsigned round;  // barriers passed
     unsigned asks;   // asks for a plan up to the last barrier (a cluster's first thread)
     int csize;       // CTAs of a cluster
+    int polls;       // of a waiting CTA before it gives up
 
     // All CTAs of the team meet; raised: the thread asked for a list build.
     // Returns the outcome of the duty.  The CTAs of a cluster tell one another
@@ -2447,14 +2446,16 @@ struct Team {
                     }
                 } else if (threadIdx.x == 0) {
                     unsigned long long v = 0;
-                    int polls = 0;
+                    int n = 0;
                     do {
                         asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&ts->open) : "memory");
-                    } while ((unsigned)(v >> 34) != (round & 0x3fffffffu) && ++polls < kTeamPolls);
+                    } while ((unsigned)(v >> 34) != (round & 0x3fffffffu) && ++n < polls);
                     asks = (unsigned)(v >> 2);
                     sh_info = (unsigned)v & 3u;
                     if ((unsigned)(v >> 34) != (round & 0x3fffffffu)) {
-                        for (int i = 0; i < A.n_slots; i++) atomicOr(&A.S[i].flags, kFlagListCorrupt);
+                        for (int i = 0; i < A.n_slots; i++)
+                            if (ld_volatile(&A.S[i].active) && !(ld_volatile(&A.S[i].flags) & kFlagFatal))
+                                atomicOr(&A.S[i].flags, kFlagWaitExpired);
                         sh_info = kTeamStop;
                     }
                 }
@@ -2506,14 +2507,15 @@ __device__ __forceinline__ bool team_stage(const BatchArgs &A, Team &team, Span 
 
 template <int D, typename FT, int KIND>
 __global__ void __maxnreg__(128)
-    k_steps(const __grid_constant__ BatchArgs A, TeamSync *ts, int steps, int csize, int motor, int rigid)
+    k_steps(const __grid_constant__ BatchArgs A, TeamSync *ts, int steps, int csize, int motor, int rigid, int polls)
 {
-    Team team{ts, 0, 0, csize};
+    Team team{ts, 0, 0, csize, polls};
     const Span sp = bead_span(A);
     // the CTAs of a cluster are scheduled together but start one by one: a
     // CTA's shared memory may be written by another only once it runs
     cluster_sync();
     unsigned info = team.sync(A, kDutyStart);
+    if (info & kTeamStop) return;
     bool raised = false;
     for (int k = 0; k < steps; k++) {
         if ((info & kTeamLists) && !team_lists<D, 0>(A, team, sp)) return;

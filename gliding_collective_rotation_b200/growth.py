@@ -39,6 +39,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
+from ._lib import FLAG_WAIT_EXPIRED
 from .batch import Batch
 from .engine import wca_params
 
@@ -203,6 +204,8 @@ def init_grow(specs, settings=None, constants=None, device=None, max_calls=1_000
                 batch.engine.call_begin_many(slots, left, batch._dts())
                 batch.run(max(left))
             for i, s in enumerate(sts):
+                if s["flags"] & FLAG_WAIT_EXPIRED:
+                    raise RuntimeError(f"system {i} stopped in the middle of a step")
                 if s["flags"] & 2:
                     raise FloatingPointError(f"system {i}: non-finite state while growing")
             t += np.where(growing, elapsed, 0.0)

@@ -39,7 +39,7 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
-from ._lib import FLAG_CELL_OVERFLOW, FLAG_LIST_OVERFLOW, GcrError
+from ._lib import FLAG_CELL_OVERFLOW, FLAG_LIST_OVERFLOW, FLAG_WAIT_EXPIRED, GcrError
 from .batch import MAX_DEPTH, MAX_LIST_DEPTH, OVERFLOW, default_depth, default_list_depth
 from .engine import Engine, SystemState
 from .workloads import SystemSpec, make_system
@@ -326,6 +326,9 @@ class Server:
             # resumes from there once the cells have grown
             n_done = st["steps_done"]
             lv.dt = st["dt"]
+            if st["flags"] & FLAG_WAIT_EXPIRED:
+                finished.append(s)  # stopped in the middle of a step: it cannot go on
+                continue
             if st["flags"] & OVERFLOW:
                 overflow = True
                 if lv.relaxing:

@@ -50,7 +50,7 @@ import numpy as np
 import torch
 
 from . import config as _default_config
-from ._lib import FLAG_CELL_OVERFLOW, FLAG_LIST_OVERFLOW, GcrError
+from ._lib import FLAG_CELL_OVERFLOW, FLAG_LIST_OVERFLOW, FLAG_WAIT_EXPIRED, GcrError
 from .batch import MAX_DEPTH, MAX_LIST_DEPTH, cell_scale, default_depth, default_list_depth
 from .engine import Engine, SystemParams, SystemState, default_config, footprint
 
@@ -239,6 +239,13 @@ def _gpu_state(pop, sim, dim, precision, params, srk_order=2):
     return g
 
 
+def _refuse_torn(g):
+    """The step stopped half way (the wait of its CTAs for one another ran
+    out): nothing is handed back, and the next call takes a new context."""
+    g.key = None
+    raise GcrError(-5, "the step stopped half way: the populations are as before the call")
+
+
 def SRK2_force_calc(pops, status, sim):
     """Stochastic Runge-Kutta 2nd-order update (Branka and Heyes, PRE 60:2381,
     1999) of one bead-spring-chain population on the GPU."""
@@ -330,6 +337,8 @@ def SRK2_force_calc(pops, status, sim):
             # time-limited: check between graphs whether the system is done
             eng.run(left if left >= 0 else (1 << 62), sync_every=1)
         res = eng.status(st.slot)
+        if res['flags'] & FLAG_WAIT_EXPIRED:
+            _refuse_torn(g)
         done += int(res['steps_done'])
         elapsed += res['dt_used']
         dt = res['dt']
@@ -536,6 +545,8 @@ def _srk2_populations(pops, status, sim, srk_order):
         flags = 0
         for r in sts:
             flags |= r['flags']
+        if flags & FLAG_WAIT_EXPIRED:
+            _refuse_torn(g)
         grow_cells = bool(flags & FLAG_CELL_OVERFLOW) and eng.cfg.cell_depth < MAX_DEPTH
         grow_lists = bool(flags & FLAG_LIST_OVERFLOW) and eng.cfg.list_depth < MAX_LIST_DEPTH
         if not (grow_cells or grow_lists) or done == max_steps or (max_dt_usable >= 0 and elapsed >= max_dt_usable):

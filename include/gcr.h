@@ -74,6 +74,9 @@ extern "C" {
 #define GCR_FLAG_LIST_CORRUPT 8    /* an inconsistent cell or neighbour list was detected and not used */
 #define GCR_FLAG_LIST_OVERFLOW 16  /* more list partners of a bead than list_depth */
 #define GCR_FLAG_SERIES_FULL 32    /* the order-parameter series buffer was full (rows dropped; not fatal) */
+#define GCR_FLAG_WAIT_EXPIRED 64   /* the CTAs of the one-kernel steps waited too long for one another: parts of
+                                      the system may be a step apart.  gcr_call_begin refuses it
+                                      (GCR_ERR_STATE) until it is evicted and admitted again */
 
 typedef struct gcr_ctx gcr_ctx;
 
