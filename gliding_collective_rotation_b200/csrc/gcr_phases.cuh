@@ -2092,10 +2092,13 @@ __device__ __forceinline__ bool rigid_tiles(const BatchArgs &A, Span sp)
         const double s2 = sqrt(2.0 * p.D * dt);
         const double rest = p.rest[c];
         const double half_clm1 = (double)(len - 1) / 2.0;
+        // (the contraction is written out: k_rigid and k_steps are compiled apart
+        // and must round it alike)
         auto upd = [&](int b, int i) {
-            double u = dt_over_r * (double)frc[(size_t)b * D + i];
-            if (s2 != 0.0) u += s2 * (double)xs[(size_t)b * D + i];
-            return u;
+            const double F = (double)frc[(size_t)b * D + i];
+            if (s2 == 0.0) return mul_rn(dt_over_r, F);
+            const double xi = (double)xs[(size_t)b * D + i];
+            return sizeof(FT) == 8 ? fma(s2, xi, mul_rn(dt_over_r, F)) : fma(dt_over_r, F, mul_rn(s2, xi));
         };
         const double *x0 = prev + (size_t)b0 * D;
         // pass 1: moment of inertia, mean update, centre, end-to-end vector
