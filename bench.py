@@ -460,9 +460,11 @@ def run_gpu(args):
         ev0 = torch.cuda.Event(enable_timing=True)
         ev1 = torch.cuda.Event(enable_timing=True)
         torch.cuda.nvtx.range_push("timed")
+        launches = eng.launches()
         ev0.record(eng.stream)
         batch.run(args.steps)
         ev1.record(eng.stream)
+        launches = eng.launches() - launches
         torch.cuda.nvtx.range_pop()
         ev1.synchronize()
         clk = clocks.stop()
@@ -679,13 +681,7 @@ def run_gpu(args):
         "one_context": dict(one_context, note="the same steps in one context, device-timed; the per-kernel "
                             "profile of `roofline` is of this context") if split else None,
         "e2e": e2e, "roofline": roofline, "clocks": clk,
-        # (per context: each context launches the whole sequence)
-        "gpu_launches": sum(count_launches(args, [specs[i] for i in part], bool(groups),
-                                           bool(getattr(specs, "motors", ())),
-                                           (args.ctas_per_sm or args.split_ctas_per_sm) if split
-                                           else args.ctas_per_sm)
-                            for part in (context_parts([sp.n for sp in specs], max(2, args.contexts), groups)
-                                         if split else [range(len(specs))])),
+        "gpu_launches": tc.launches if split else launches,
     }
     if fp64 is not None:
         line["fp64"] = fp64
@@ -718,27 +714,6 @@ def split_by_beads(sizes, k):
         cuts.append(min(max(c, cuts[-1] + 1), n - (k - q)))
     cuts.append(n)
     return cuts
-
-
-def count_launches(args, specs, coupled, motors, ctas_per_sm):
-    """Kernel launches of ``args.steps`` steps of one context (csrc/gcr_abi.cu):
-    the run-start check, then one kernel for up to 512 steps while every tile
-    has a CTA of its own (592 of 128 threads, half with coupled populations, 16
-    in a context of several), else graphs of steps_per_graph steps with, per step, two list builds of two
-    kernels, three of per-system work, two stages and the update, two pair
-    kernels (none where the stages sum the pair forces: 2D mixed precision in a
-    context alone and pair_mode 1, without coupled populations), two sorts in pair_mode 2 and two
-    motor kernels with motor populations."""
-    steps = args.steps_per_graph * math.ceil(args.steps / args.steps_per_graph)
-    tiles = sum(-(-sp.n // args.block_beads) for sp in specs)
-    limit = 148 * (65536 // (128 * args.block_beads)) // (2 if coupled else 1)
-    limit = 16 if ctas_per_sm > 0 else max(limit, 8)
-    if ctas_per_sm >= 0 and (coupled or args.pair_mode != 2) and tiles <= limit:
-        return 1 + -(-steps // 512)
-    mode = 0 if coupled else args.pair_mode
-    own = not coupled and mode != 2 and (mode == 1 or (ctas_per_sm <= 0 and specs[0].dim == 2 and args.precision == "mixed"))
-    per_step = 10 + (0 if own else 2) + (2 if mode == 2 else 0) + (2 if motors else 0)
-    return 2 + per_step * steps
 
 
 def context_parts(sizes, k, groups=()):
@@ -791,6 +766,7 @@ class SplitContexts:
             hb.run_checked(max(args.warmup, 1))
             self.parts.append(hb)
         self.regrows = 0
+        self.launches = 0  # step kernels of the timed steps, over the contexts
 
     def statuses(self):
         return [st for hb in self.parts for st in hb.statuses()]
@@ -810,6 +786,7 @@ class SplitContexts:
             ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             barrier()
             torch.cuda.nvtx.range_push("timed_contexts")
+            launches = -sum(hb.engine.launches() for hb in self.parts)
             ev0.record(s0)
             for st in streams[1:]:
                 st.wait_event(ev0)
@@ -825,6 +802,7 @@ class SplitContexts:
             torch.cuda.synchronize()
             barrier()
             ms = ev0.elapsed_time(ev1)
+            self.launches = launches + sum(hb.engine.launches() for hb in self.parts)
             over = [hb.overflowed() for hb in self.parts]
             if not any_rank(any(over)) or attempt == 3:
                 return ms, self.statuses()

@@ -82,6 +82,7 @@ SIGNATURES = {
     "gcr_get_status": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(Status)]),
     "gcr_get_statuses": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_int32), C.POINTER(Status)]),
     "gcr_count_active": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32)]),
+    "gcr_launches": (C.c_int, [C.c_void_p, C.POINTER(C.c_int64)]),
     "gcr_synchronize": (C.c_int, [C.c_void_p]),
     "gcr_profile_steps": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_float)]),
     "gcr_order_params": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double)]),

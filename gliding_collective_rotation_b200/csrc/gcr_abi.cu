@@ -184,6 +184,8 @@ struct gcr_ctx {
     int64_t x_rows = 0;        // rows allocated (the slot stride of xnbr)
     void *observe = nullptr;   // k_observe of the context's precision
     bool pdl = true;           // programmatic dependent launch of the step kernels
+    int64_t launched = 0;      // step kernels queued, those of the launched graphs among them
+    int64_t graph_kernels = 0; // ... of one graph
     bool tiles_dirty = true;
 };
 
@@ -615,6 +617,7 @@ int launch_args(gcr_ctx *c, void *fn, int grid, int block, size_t smem, void **a
     lc.attrs = at;
     lc.numAttrs = 1;
     GCR_CUDA(cudaLaunchKernelExC(&lc, fn, a));
+    c->launched++;
     return GCR_OK;
 }
 
@@ -793,7 +796,10 @@ int build_graph(gcr_ctx *c)
     cudaGraph_t g = nullptr;
     GCR_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int rc = GCR_OK;
+    const int64_t before = c->launched;
     for (int s = 0; s < c->cfg.steps_per_graph && rc == GCR_OK; s++) rc = enqueue_step(c);
+    c->graph_kernels = c->launched - before;
+    c->launched = before;
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (rc != GCR_OK) {
         if (g) cudaGraphDestroy(g);
@@ -884,6 +890,7 @@ int launch_steps(gcr_ctx *c, int64_t steps)
     lc.attrs = at;
     lc.numAttrs = one ? 1 : 2;
     GCR_CUDA(cudaLaunchKernelExC(&lc, c->ks.steps[kind], a));
+    c->launched++;
     return GCR_OK;
 }
 
@@ -1598,6 +1605,7 @@ int gcr_run(gcr_ctx *c, int64_t max_steps, int32_t sync_every)
             if ((rc = run_one_kernel(c, spg))) return rc;
         } else {
             GCR_CUDA(cudaGraphLaunch(c->graph, c->stream));
+            c->launched += c->graph_kernels;
             for (int64_t &q : c->attempts) q += spg;
         }
         if (sync_every > 0 && (g + 1) % sync_every == 0 && g + 1 < graphs) {
@@ -1685,6 +1693,13 @@ int gcr_synchronize(gcr_ctx *c)
 {
     if (!c) return fail(GCR_ERR_BAD_ARG, "null context");
     GCR_CUDA(cudaStreamSynchronize(c->stream));
+    return GCR_OK;
+}
+
+int gcr_launches(gcr_ctx *c, int64_t *n_out)
+{
+    if (!c || !n_out) return fail(GCR_ERR_BAD_ARG, "null argument");
+    *n_out = c->launched;
     return GCR_OK;
 }
 

@@ -345,6 +345,12 @@ class Engine:
         check(self.lib.gcr_profile_steps(self._ctx, int(n_steps), out))
         return np.array(out[:], dtype=np.float64)
 
+    def launches(self):
+        """Step kernels queued since the context was created."""
+        n = C.c_int64()
+        check(self.lib.gcr_launches(self._ctx, C.byref(n)))
+        return n.value
+
     def count_active(self):
         n = C.c_int32()
         check(self.lib.gcr_count_active(self._ctx, C.byref(n)))

@@ -272,6 +272,10 @@ GCR_API int gcr_get_statuses(gcr_ctx *ctx, int32_t n, const int32_t *slots, gcr_
 /* Number of armed systems still running (synchronises the stream). */
 GCR_API int gcr_count_active(gcr_ctx *ctx, int32_t *n_out);
 GCR_API int gcr_synchronize(gcr_ctx *ctx);
+/* Step kernels queued by gcr_run and gcr_profile_steps since the context was
+ * created, each kernel of a launched graph counted (host; no counterpart in
+ * the reference). */
+GCR_API int gcr_launches(gcr_ctx *ctx, int64_t *n_out);
 /* Run `n_steps` steps launching the step kernels one by one (not through
  * the graph) with CUDA events between groups on the context stream;
  * ms_out[0..6] receive the total milliseconds of: cell list of pos (scans and
