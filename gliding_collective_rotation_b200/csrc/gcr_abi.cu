@@ -154,6 +154,7 @@ struct gcr_ctx {
     int *d_err = nullptr;
     double *d_out = nullptr;
     int64_t max_bead_tiles = 0, max_cell_tiles = 0;
+    int64_t list_cells = 0, fixed_beads = 0;  // of the resident systems: what list builds visit beside the bead tiles
     // host mirrors
     std::vector<Slot> slots;
     std::vector<SysP> hP;
@@ -260,6 +261,7 @@ int rebuild_tiles(gcr_ctx *c)
     c->h_cell_tiles.clear();
     c->h_row_prefix.assign(c->slots.size() + 1, 0);
     int64_t rows = 0;
+    c->list_cells = c->fixed_beads = 0;
     const int tb = c->cfg.block_beads, tcl = c->cfg.block_cells;
     for (int s = 0; s < (int)c->slots.size(); s++) {
         const Slot &sl = c->slots[s];
@@ -267,6 +269,9 @@ int rebuild_tiles(gcr_ctx *c)
         // a fixed population never moves: only the list kernels visit it
         if (!c->hP[s].fixed)
             for (int64_t b = 0; b < sl.desc.n_beads; b += tb) c->h_bead_tiles.push_back(Tile{s, (int32_t)b});
+        else
+            c->fixed_beads += sl.desc.n_beads;
+        if (sl.desc.calc_wca) c->list_cells += sl.n_cells;
         if (sl.desc.calc_wca)
             for (int64_t q = 0; q < sl.n_cells; q += tcl) c->h_cell_tiles.push_back(Tile{s, (int32_t)q});
     }
@@ -812,6 +817,13 @@ int build_graph(gcr_ctx *c)
     return GCR_OK;
 }
 
+// Cells a CTA of the one-kernel steps may have to zero at a list build, a bead of
+// a fixed population that it bins counted as kFixedBeadCells.  With a build in
+// every step or more, us a step by launches and in one kernel (B200): 1000 beads,
+// 8 CTAs, 3D 56k cells a CTA 31, 29; 97k 33, 36; 155k 31, 45; 778k 32, 150;
+// 100 beads beside 10k fixed ones 44, 34; 15k 47, 50; 20k 51, 62; 200k 47, 327.
+constexpr int64_t kTeamCells = 64 * 1024, kFixedBeadCells = 3;
+
 // which k_steps a batch needs
 int steps_kind(const gcr_ctx *c)
 {
@@ -838,6 +850,9 @@ bool one_kernel_steps(gcr_ctx *c)
     // a context told to leave room for others (ctas_per_sm) launches: cooperative
     // kernels that do not fit together run one after another
     if (c->cfg.ctas_per_sm > 0 && tiles > 16) return false;
+    // a list build is for these CTAs alone: they zero the cells of a dilute box
+    // and bin a fixed population, which a launch spreads over the device
+    if (c->list_cells + kFixedBeadCells * c->fixed_beads > kTeamCells * std::max<int64_t>(tiles, 1)) return false;
     // no more than the registers allow fit; a portable cluster always does
     // (the device is asked only where that leaves it open: a query takes longer
     // than a step)
@@ -1122,7 +1137,10 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     c->grid_pair = kernel_grid(c, c->ks.pair0, cfg.block_beads, c->max_bead_tiles, c->pair_smem);
     c->grid_bin = kernel_grid(c, c->ks.bin0, cfg.block_beads, c->max_bead_tiles);
     c->grid_sort = kernel_grid(c, c->ks.sort, cfg.block_cells, c->max_cell_tiles);
-    c->grid_build = kernel_grid(c, c->ks.build0, cfg.block_beads, c->max_bead_tiles, c->build_smem);
+    // (a dilute box has far more cells to zero than beads: 1000 beads in 6.2
+    // million cells 157 us a step with a CTA for each of their tiles, 65 so)
+    c->grid_build = kernel_grid(c, c->ks.build0, cfg.block_beads, std::max(c->max_bead_tiles, c->max_cell_tiles / 8),
+                                c->build_smem);
     c->grid_sys = (int)((S + 127) / 128);
     c->steps_smem = steps_smem(c, cfg.block_beads, std::min(kTeamBuildCap, a.build_cap));
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return cleanup(fail(GCR_ERR_CUDA, "initialisation"));
