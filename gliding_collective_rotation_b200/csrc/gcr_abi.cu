@@ -130,7 +130,7 @@ struct gcr_ctx {
     Tile *d_bead_tiles = nullptr;
     Tile *d_cell_tiles = nullptr;
     int *d_row_prefix = nullptr;  // row tiles of the cell-staged pair kernel per slot, prefix [S + 1]
-    int *d_ntiles = nullptr;  // [0] bead tiles, [1] cell tiles
+    int *d_ntiles = nullptr;  // [0] bead tiles, [1] cell tiles, [2] slots in use, [3] BatchArgs::duty_done
     uint8_t *topo = nullptr;
     int *cnt[2] = {nullptr, nullptr};  // beads per cell, in turns (SysS::turn)
     int *items = nullptr;
@@ -154,6 +154,7 @@ struct gcr_ctx {
     int *d_err = nullptr;
     double *d_out = nullptr;
     int64_t max_bead_tiles = 0, max_cell_tiles = 0;
+    int used_slots = 0;  // up to the last resident system's
     int64_t list_cells = 0, fixed_beads = 0;  // of the resident systems: what list builds visit beside the bead tiles
     // host mirrors
     std::vector<Slot> slots;
@@ -285,7 +286,9 @@ int rebuild_tiles(gcr_ctx *c)
                              c->stream));
     if ((int64_t)c->h_bead_tiles.size() > c->max_bead_tiles || (int64_t)c->h_cell_tiles.size() > c->max_cell_tiles)
         return fail(GCR_ERR_CAPACITY, "tile table capacity exceeded");
-    int nt[2] = {(int)c->h_bead_tiles.size(), (int)c->h_cell_tiles.size()};
+    c->used_slots = (int)c->slots.size();
+    while (c->used_slots > 0 && !c->slots[c->used_slots - 1].used) c->used_slots--;
+    int nt[3] = {(int)c->h_bead_tiles.size(), (int)c->h_cell_tiles.size(), c->used_slots};
     if (nt[0]) GCR_CUDA(cudaMemcpyAsync(c->d_bead_tiles, c->h_bead_tiles.data(), nt[0] * sizeof(Tile),
                                         cudaMemcpyHostToDevice, c->stream));
     if (nt[1]) GCR_CUDA(cudaMemcpyAsync(c->d_cell_tiles, c->h_cell_tiles.data(), nt[1] * sizeof(Tile),
@@ -636,7 +639,10 @@ int launch(gcr_ctx *c, void *fn, int grid, int block, size_t smem = 0)
 int launch_duty(gcr_ctx *c, int duty)
 {
     void *a[] = {&c->args, &duty};
-    return launch_args(c, c->ks.duty, 1, 1024, 0, a);
+    // the dt rule over many SMs (its square roots and divisions), the end of the
+    // step in few CTAs, as the last of them makes the plan
+    const int block = duty == kDutyDt ? 128 : 1024, ctas = ((int)c->slots.size() + block - 1) / block;
+    return launch_args(c, c->ks.duty, duty == kDutyDt || duty == kDutyEnd ? ctas : 1, block, 0, a);
 }
 
 // one stage's neighbour lists, of the systems that the plan took: bin, (for the cell-staged pair forces) per-cell sort, build
@@ -850,6 +856,10 @@ bool one_kernel_steps(gcr_ctx *c)
     // a context told to leave room for others (ctas_per_sm) launches: cooperative
     // kernels that do not fit together run one after another
     if (c->cfg.ctas_per_sm > 0 && tiles > 16) return false;
+    // the per-system work is one CTA's: a thread a slot, or its chains of loads
+    // come in turn (systems of 30 beads, by launches and in one kernel: 64 36, 30;
+    // 128 40, 40; 256 46, 56; 400 51, 71 us a step)
+    if (c->used_slots > bb) return false;
     // a list build is for these CTAs alone: they zero the cells of a dilute box
     // and bin a fixed population, which a launch spreads over the device
     if (c->list_cells + kFixedBeadCells * c->fixed_beads > kTeamCells * std::max<int64_t>(tiles, 1)) return false;
@@ -1034,7 +1044,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     e = e ? e : cudaMalloc(&c->dS, sizeof(SysS) * S);
     e = e ? e : cudaMalloc(&c->d_bead_tiles, sizeof(Tile) * c->max_bead_tiles);
     e = e ? e : cudaMalloc(&c->d_cell_tiles, sizeof(Tile) * c->max_cell_tiles);
-    e = e ? e : cudaMalloc(&c->d_ntiles, sizeof(int) * 2);
+    e = e ? e : cudaMalloc(&c->d_ntiles, sizeof(int) * 4);
     e = e ? e : cudaMalloc(&c->d_row_prefix, sizeof(int) * (size_t)(S + 1));
     e = e ? e : cudaMemsetAsync(c->d_row_prefix, 0, sizeof(int) * (size_t)(S + 1), c->stream);
     e = e ? e : cudaMalloc(&c->topo, (size_t)cfg.bead_capacity);
@@ -1060,7 +1070,7 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
         return cleanup(fail(e == cudaErrorMemoryAllocation ? GCR_ERR_OOM : GCR_ERR_CUDA,
                             std::string("device allocation: ") + cudaGetErrorString(e)));
     cudaMemsetAsync(c->dS, 0, sizeof(SysS) * S, c->stream);
-    cudaMemsetAsync(c->d_ntiles, 0, sizeof(int) * 2, c->stream);
+    cudaMemsetAsync(c->d_ntiles, 0, sizeof(int) * 4, c->stream);
     for (int *cnt : c->cnt) cudaMemsetAsync(cnt, 0, sizeof(int) * cells_alloc, c->stream);
     cudaMemsetAsync(c->ncount, 0, sizeof(int) * (size_t)cfg.bead_capacity, c->stream);
     cudaMemsetAsync(c->img, 0, sizeof(int) * (size_t)cfg.bead_capacity * cfg.dim, c->stream);
@@ -1079,6 +1089,8 @@ int gcr_create(const gcr_config *cfg_in, void *cuda_stream, gcr_ctx **out)
     a.n_bead_tiles = c->d_ntiles;
     a.cell_tiles = c->d_cell_tiles;
     a.n_cell_tiles = c->d_ntiles + 1;
+    a.n_used = c->d_ntiles + 2;
+    a.duty_done = reinterpret_cast<unsigned *>(c->d_ntiles + 3);
     a.topo = c->topo;
     a.cnt0 = c->cnt[0];
     a.cnt1 = c->cnt[1];

@@ -329,10 +329,11 @@ static __device__ __noinline__ int plan_lists(const BatchArgs &A)
     if (threadIdx.x < 3) carry[threadIdx.x] = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int base = 0; base < A.n_slots; base += blockDim.x) {
+    const int used = *A.n_used;
+    for (int base = 0; base < used; base += blockDim.x) {
         const int i = base + threadIdx.x;
         int v[3] = {0, 0, 0};
-        if (i < A.n_slots) {
+        if (i < used) {
             const SysP &p = A.P[i];
             const SysS &st = A.S[i];
             bool part = false;
@@ -509,15 +510,12 @@ __device__ __forceinline__ bool sys_end(const BatchArgs &A, int i)
 }
 
 // The per-system work between two kernels of a step, done by one CTA: the list
-// plan, the dt rule, the step bookkeeping with the next step's plan.  That
+// plan, and the step bookkeeping with the next step's plan.  That
 // plan is still to be carried out when a run ends: the next run starts by
 // taking it back, and plans anew.
 static __device__ __noinline__ void step_duty(const BatchArgs &A, int duty)
 {
-    if (duty == kDutyDt) {
-        for (int i = threadIdx.x; i < A.n_slots; i += blockDim.x) sys_dt(A, i);
-        return;
-    }
+    const int used = *A.n_used;
     if (duty == kDutyStart) {
         const int m = min(A.work[0], A.n_slots);
         for (int k = threadIdx.x; k < m; k += blockDim.x) {
@@ -529,9 +527,9 @@ static __device__ __noinline__ void step_duty(const BatchArgs &A, int duty)
         __syncthreads();
     }
     // the plan is made only when some system asks for a build: most stages
-    // none does
-    bool ask = false;
-    for (int i = threadIdx.x; i < A.n_slots; i += blockDim.x) {
+    // none does (with more systems than threads one usually does)
+    bool ask = used > (int)blockDim.x;
+    for (int i = threadIdx.x; i < used && !ask; i += blockDim.x) {
         if (duty == kDutyEnd) sys_end(A, i);
         ask |= A.S[i].rebuild != 0;
     }
@@ -2363,7 +2361,7 @@ constexpr unsigned kTeamLists = 1, kTeamStop = 2;
 static __device__ __noinline__ unsigned team_duty(const BatchArgs &A, int duty, bool ask)
 {
     if (duty == kDutyDt) {
-        for (int i = threadIdx.x; i < A.n_slots; i += blockDim.x) sys_dt(A, i);
+        for (int i = threadIdx.x; i < *A.n_used; i += blockDim.x) sys_dt(A, i);
         return 0;
     }
     if (duty == kDutyStart) {
@@ -2373,7 +2371,7 @@ static __device__ __noinline__ unsigned team_duty(const BatchArgs &A, int duty, 
     }
     if (duty == kDutyEnd) {
         bool more = false;
-        for (int i = threadIdx.x; i < A.n_slots; i += blockDim.x) more |= sys_end(A, i);
+        for (int i = threadIdx.x; i < *A.n_used; i += blockDim.x) more |= sys_end(A, i);
         if (!__syncthreads_or(more)) return kTeamStop;
     }
     return ask && plan_lists(A) > 0 ? kTeamLists : 0;
