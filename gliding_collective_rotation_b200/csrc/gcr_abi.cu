@@ -642,7 +642,7 @@ int launch_duty(gcr_ctx *c, int duty)
     // the dt rule over many SMs (its square roots and divisions), the end of the
     // step in few CTAs, as the last of them makes the plan
     const int block = duty == kDutyDt ? 128 : 1024, ctas = ((int)c->slots.size() + block - 1) / block;
-    return launch_args(c, c->ks.duty, duty == kDutyDt || duty == kDutyEnd ? ctas : 1, block, 0, a);
+    return launch_args(c, c->ks.duty, duty == kDutyStart ? 1 : ctas, block, 0, a);
 }
 
 // one stage's neighbour lists, of the systems that the plan took: bin, (for the cell-staged pair forces) per-cell sort, build

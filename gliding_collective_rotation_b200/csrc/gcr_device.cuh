@@ -178,6 +178,13 @@ __device__ __forceinline__ void set_predictor(const SysP &p, SysS &s, bool mixed
     set_step_const(s, mixed, kSPredNoise, sqrt(2.0 * s.dt * p.D));
 }
 
+// a system asks for a list build: one that has finished, was never armed or has
+// been stopped does not, whatever its flag says
+__host__ __device__ __forceinline__ bool asks_build(const SysP &p, const SysS &s)
+{
+    return s.rebuild && s.active && !(s.flags & kFlagFatal) && p.calc_wca && !p.fixed;
+}
+
 struct Tile {
     int32_t sys;
     int32_t begin;

@@ -339,7 +339,7 @@ static __device__ __noinline__ int plan_lists(const BatchArgs &A)
             bool part = false;
             if (p.calc_wca && !(st.flags & kFlagFatal)) {
                 if (p.grp_n == 0) {
-                    part = st.active && st.rebuild;
+                    part = asks_build(p, st);
                 } else {
                     // coupled populations rebuild together: their cross lists
                     // read one another's cells.  Only moving, running members
@@ -349,8 +349,7 @@ static __device__ __noinline__ int plan_lists(const BatchArgs &A)
                     for (int k = 0; k < p.grp_n && k < kMaxPops; k++) {
                         const int m = p.grp[k];
                         if (m < 0 || m >= A.n_slots) continue;
-                        const SysS &sm = A.S[m];
-                        any |= !A.P[m].fixed && sm.active && sm.rebuild && !(sm.flags & kFlagFatal);
+                        any |= asks_build(A.P[m], A.S[m]);
                     }
                     part = any && (p.fixed || st.active);
                 }
@@ -509,6 +508,15 @@ __device__ __forceinline__ bool sys_end(const BatchArgs &A, int i)
     return more;
 }
 
+// the plan is made only when some system asks for a build: most stages none does
+__device__ __forceinline__ void make_plan(const BatchArgs &A, bool ask)
+{
+    if (ask)
+        plan_lists(A);
+    else if (threadIdx.x < 3)
+        A.work[threadIdx.x] = 0;
+}
+
 // The per-system work between two kernels of a step, done by one CTA: the list
 // plan, and the step bookkeeping with the next step's plan.  That
 // plan is still to be carried out when a run ends: the next run starts by
@@ -526,17 +534,12 @@ static __device__ __noinline__ void step_duty(const BatchArgs &A, int duty)
         }
         __syncthreads();
     }
-    // the plan is made only when some system asks for a build: most stages
-    // none does (with more systems than threads one usually does)
-    bool ask = used > (int)blockDim.x;
-    for (int i = threadIdx.x; i < used && !ask; i += blockDim.x) {
+    bool ask = false;
+    for (int i = threadIdx.x; i < used; i += blockDim.x) {
         if (duty == kDutyEnd) sys_end(A, i);
-        ask |= A.S[i].rebuild != 0;
+        ask |= asks_build(A.P[i], A.S[i]);
     }
-    if (__syncthreads_or(ask))
-        plan_lists(A);
-    else if (threadIdx.x < 3)
-        A.work[threadIdx.x] = 0;
+    make_plan(A, __syncthreads_or(ask));
 }
 
 // bin every bead of a flagged system into its cell (fixed-depth slots)

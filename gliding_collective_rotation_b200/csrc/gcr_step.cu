@@ -5,7 +5,7 @@
 namespace gcr {
 
 // the per-system work between two kernels of a step: one CTA, or one for each
-// 1024 slots, the last of which to end a step makes the next plan (4096 systems
+// 1024 slots, the last of which to finish makes the plan (4096 systems
 // of 30 beads 183 us a step with one CTA throughout, 16,384 of 10 522 us)
 __global__ void __launch_bounds__(1024) k_duty(const __grid_constant__ BatchArgs A, int duty)
 {
@@ -16,17 +16,21 @@ __global__ void __launch_bounds__(1024) k_duty(const __grid_constant__ BatchArgs
         if (i < used) sys_dt(A, i);
         return;
     }
-    if (duty == kDutyEnd && ctas > 1) {
+    if (duty != kDutyStart && ctas > 1) {
         if (blockIdx.x >= ctas) return;
-        if (i < used) sys_end(A, i);
+        if (duty == kDutyEnd && i < used) sys_end(A, i);
+        const int ask = __syncthreads_or(i < used && asks_build(A.P[i], A.S[i]));
         __threadfence();
         __syncthreads();
-        if (__syncthreads_or(threadIdx.x == 0 && atomicAdd(A.duty_done, 1u) + 1u < ctas)) return;
+        unsigned done = 0;
+        if (threadIdx.x == 0) done = atomicAdd(A.duty_done, 1u + (ask ? 65536u : 0u)) + 1u + (ask ? 65536u : 0u);
+        if (!__syncthreads_or((done & 65535u) == ctas)) return;
         if (threadIdx.x == 0) *A.duty_done = 0;
         __threadfence();
-        duty = kDutyPlan;
+        make_plan(A, __syncthreads_or(done >> 16));
+        return;
     }
-    if (duty == kDutyEnd && blockIdx.x > 0) return;
+    if (blockIdx.x > 0) return;
     step_duty(A, duty);
 }
 
