@@ -920,14 +920,15 @@ int launch_steps(gcr_ctx *c, int64_t steps)
 }
 
 // steps until some system's series takes its next row (at most `steps`):
-// its call's steps, plus the call's phase, reach a multiple of the interval
+// its call's steps, plus the call's phase, reach a multiple of the interval.  A
+// call that has ended, or ends before, takes none (hS: as last armed or fetched)
 int64_t steps_to_row(const gcr_ctx *c, int64_t steps)
 {
     for (size_t s = 0; s < c->slots.size(); s++) {
         const SysS &st = c->hS[s];
-        if (!c->slots[s].used || !st.series || st.series_every <= 0) continue;
-        const int64_t at = (c->attempts[s] + st.series_phase) % st.series_every;
-        steps = std::min(steps, st.series_every - at);
+        if (!c->slots[s].used || !st.series || st.series_every <= 0 || !st.active) continue;
+        const int64_t to = st.series_every - (c->attempts[s] + st.series_phase) % st.series_every;
+        if (st.max_steps < 0 || c->attempts[s] + to <= st.max_steps) steps = std::min(steps, to);
     }
     return steps;
 }
