@@ -639,10 +639,12 @@ int launch(gcr_ctx *c, void *fn, int grid, int block, size_t smem = 0)
 int launch_duty(gcr_ctx *c, int duty)
 {
     void *a[] = {&c->args, &duty};
-    // the dt rule over many SMs (its square roots and divisions), the end of the
-    // step in few CTAs, as the last of them makes the plan
-    const int block = duty == kDutyDt ? 128 : 1024, ctas = ((int)c->slots.size() + block - 1) / block;
-    return launch_args(c, c->ks.duty, duty == kDutyStart ? 1 : ctas, block, 0, a);
+    // the dt rule over several SMs (its square roots and divisions) sooner than the
+    // rest, as the plan is one CTA's
+    const int n = (int)c->slots.size(), block = duty == kDutyDt ? 128 : 1024;
+    if (duty != kDutyStart && n > (duty == kDutyDt ? 256 : 1024))
+        return launch_args(c, c->ks.duty_wide, (n + block - 1) / block, block, 0, a);
+    return launch_args(c, c->ks.duty, 1, 1024, 0, a);
 }
 
 // one stage's neighbour lists, of the systems that the plan took: bin, (for the cell-staged pair forces) per-cell sort, build

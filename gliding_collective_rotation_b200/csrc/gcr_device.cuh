@@ -179,10 +179,10 @@ __device__ __forceinline__ void set_predictor(const SysP &p, SysS &s, bool mixed
 }
 
 // a system asks for a list build: one that has finished, was never armed or has
-// been stopped does not, whatever its flag says
+// been stopped does not, whatever its flag says (every word is read at once)
 __host__ __device__ __forceinline__ bool asks_build(const SysP &p, const SysS &s)
 {
-    return s.rebuild && s.active && !(s.flags & kFlagFatal) && p.calc_wca && !p.fixed;
+    return (s.rebuild != 0) & (s.active != 0) & !(s.flags & kFlagFatal) & (p.calc_wca != 0) & (p.fixed == 0);
 }
 
 struct Tile {

@@ -29,7 +29,7 @@ struct BatchArgs {
     int build_cap; // list entries a thread of the build sorts in shared memory
     int n_slots;
     const int *n_used;    // slots up to the last resident system's: what the per-system work visits
-    unsigned *duty_done;  // CTAs of k_duty that have done their share, 0 between launches
+    unsigned *duty_done;  // CTAs of k_duty_wide that have done their share (+ 65536 each that asks for a plan)
     int64_t list_stride;
     int list_depth;
     int depth;
@@ -98,7 +98,8 @@ struct KernelSet {
     void *pair2;
     void *rigid4[4];
     void *topo;
-    void *duty;      // per-system work between two kernels of a step (kDuty...)
+    void *duty;      // per-system work between two kernels of a step (kDuty...), one CTA
+    void *duty_wide; // ... of many systems
     void *sys_mark;  // flag one resident system (or all) for a list build
     void *run_check;  // run start: flag the armed systems whose lists no longer cover their positions
     void *pair_cross[3];  // pair forces at pos / pos1 / pos2 with the other populations' (coupled systems)

@@ -287,8 +287,9 @@ __device__ __forceinline__ Span bead_span(const BatchArgs &A)
 struct Work {
     int m, n_bead, n_cell;
     const int *sys, *bead0, *cell0;
-    int *outside;
+    bool loose;  // of a build: its binning found a bead outside its box
 };
+__device__ __forceinline__ int *work_outside(const BatchArgs &A) { return A.work + 3 * A.n_slots + 5; }
 
 __device__ __forceinline__ Work work_list(const BatchArgs &A)
 {
@@ -300,7 +301,7 @@ __device__ __forceinline__ Work work_list(const BatchArgs &A)
     w.sys = q + 3;
     w.bead0 = w.sys + A.n_slots;
     w.cell0 = w.bead0 + A.n_slots + 1;
-    w.outside = A.work + (w.cell0 + A.n_slots + 1 - q);
+    w.loose = *work_outside(A) != 0;
     return w;
 }
 
@@ -318,6 +319,14 @@ __device__ __forceinline__ int work_owner(const int *pre, int m, int i)
     return lo;
 }
 
+// slots a CTA visits in the per-system work: those in use, or all of them where
+// each has a thread anyway (an empty one is not active), which saves a load that
+// everything else would wait for
+__device__ __forceinline__ int slots_used(const BatchArgs &A)
+{
+    return A.n_slots <= (int)blockDim.x ? A.n_slots : *A.n_used;
+}
+
 // one CTA: compact the systems that take part in a list build now; returns
 // how many there are
 static __device__ __noinline__ int plan_lists(const BatchArgs &A)
@@ -329,7 +338,7 @@ static __device__ __noinline__ int plan_lists(const BatchArgs &A)
     if (threadIdx.x < 3) carry[threadIdx.x] = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int used = *A.n_used;
+    const int used = slots_used(A);
     for (int base = 0; base < used; base += blockDim.x) {
         const int i = base + threadIdx.x;
         int v[3] = {0, 0, 0};
@@ -404,7 +413,7 @@ static __device__ __noinline__ int plan_lists(const BatchArgs &A)
         q[0] = carry[0];
         q[1] = carry[1];
         q[2] = carry[2];
-        wc[A.n_slots + 1] = 0;
+        *work_outside(A) = 0;
         wb[carry[0]] = carry[1];
         wc[carry[0]] = carry[2];
     }
@@ -523,7 +532,7 @@ __device__ __forceinline__ void make_plan(const BatchArgs &A, bool ask)
 // taking it back, and plans anew.
 static __device__ __noinline__ void step_duty(const BatchArgs &A, int duty)
 {
-    const int used = *A.n_used;
+    const int used = slots_used(A);
     if (duty == kDutyStart) {
         const int m = min(A.work[0], A.n_slots);
         for (int k = threadIdx.x; k < m; k += blockDim.x) {
@@ -563,7 +572,7 @@ __device__ __forceinline__ void bin_tiles(const BatchArgs &A, Span sp)
         cell_of<D>(p, x, ci);
 #pragma unroll
         for (int i = 0; i < D; i++)
-            if (!(x[i] >= 0.0 && x[i] <= p.L)) *w.outside = 1;
+            if (!(x[i] >= 0.0 && x[i] <= p.L)) *work_outside(A) = 1;
         const int64_t gc = p.cell_off + ((int64_t)ci[2] * p.nc + ci[1]) * p.nc + ci[0];
         const int slot = atomicAdd(cell_counts(A, s.turn) + gc, 1);
         if (slot < A.depth)
@@ -896,7 +905,7 @@ __device__ __forceinline__ void build_tiles(const BatchArgs &A, Span sp)
         const int c0 = (t - w.cell0[k]) * A.tile_cells, c1 = min(c0 + A.tile_cells, p.n_cells);
         for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) other[p.cell_off + c] = 0;
     }
-    if (w.n_bead > 0 && *w.outside)
+    if (w.loose)
         build_lists_loose<D, WHICH>(A, sp);
     else
         build_lists<D, WHICH, false>(A, w, sp);
@@ -2364,7 +2373,7 @@ constexpr unsigned kTeamLists = 1, kTeamStop = 2;
 static __device__ __noinline__ unsigned team_duty(const BatchArgs &A, int duty, bool ask)
 {
     if (duty == kDutyDt) {
-        for (int i = threadIdx.x; i < *A.n_used; i += blockDim.x) sys_dt(A, i);
+        for (int i = threadIdx.x, n = slots_used(A); i < n; i += blockDim.x) sys_dt(A, i);
         return 0;
     }
     if (duty == kDutyStart) {
@@ -2374,7 +2383,7 @@ static __device__ __noinline__ unsigned team_duty(const BatchArgs &A, int duty, 
     }
     if (duty == kDutyEnd) {
         bool more = false;
-        for (int i = threadIdx.x; i < *A.n_used; i += blockDim.x) more |= sys_end(A, i);
+        for (int i = threadIdx.x, n = slots_used(A); i < n; i += blockDim.x) more |= sys_end(A, i);
         if (!__syncthreads_or(more)) return kTeamStop;
     }
     return ask && plan_lists(A) > 0 ? kTeamLists : 0;

@@ -4,34 +4,42 @@
 
 namespace gcr {
 
-// the per-system work between two kernels of a step: one CTA, or one for each
-// 1024 slots, the last of which to finish makes the plan (4096 systems
-// of 30 beads 183 us a step with one CTA throughout, 16,384 of 10 522 us)
+// one CTA: the per-system work between two kernels of a step
 __global__ void __launch_bounds__(1024) k_duty(const __grid_constant__ BatchArgs A, int duty)
 {
     pdl_wait();
-    const int used = *A.n_used, i = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned ctas = max(1, (used + (int)blockDim.x - 1) / (int)blockDim.x);
     if (duty == kDutyDt) {
-        if (i < used) sys_dt(A, i);
+        for (int i = threadIdx.x; i < A.n_slots; i += blockDim.x) sys_dt(A, i);
         return;
     }
-    if (duty != kDutyStart && ctas > 1) {
-        if (blockIdx.x >= ctas) return;
-        if (duty == kDutyEnd && i < used) sys_end(A, i);
-        const int ask = __syncthreads_or(i < used && asks_build(A.P[i], A.S[i]));
-        __threadfence();
-        __syncthreads();
-        unsigned done = 0;
-        if (threadIdx.x == 0) done = atomicAdd(A.duty_done, 1u + (ask ? 65536u : 0u)) + 1u + (ask ? 65536u : 0u);
-        if (!__syncthreads_or((done & 65535u) == ctas)) return;
-        if (threadIdx.x == 0) *A.duty_done = 0;
-        __threadfence();
-        make_plan(A, __syncthreads_or(done >> 16));
-        return;
-    }
-    if (blockIdx.x > 0) return;
     step_duty(A, duty);
+}
+
+// ... of many systems: a thread a slot, and the last CTA to finish makes the plan
+// (4096 systems of 30 beads 183 us a step with one CTA, 130 so; 16,384 of 10 522
+// and 276).  A kernel of its own: with this in k_duty a step of few systems, whose
+// launches begin with cold instruction caches, took 0.8 us more.
+__global__ void __launch_bounds__(1024) k_duty_wide(const __grid_constant__ BatchArgs A, int duty)
+{
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (duty == kDutyDt) {
+        if (i < A.n_slots) sys_dt(A, i);
+        return;
+    }
+    const int used = *A.n_used;
+    const unsigned ctas = max(1, (used + (int)blockDim.x - 1) / (int)blockDim.x);
+    if (blockIdx.x >= ctas) return;
+    if (duty == kDutyEnd && i < used) sys_end(A, i);
+    const int ask = __syncthreads_or(i < used && asks_build(A.P[i], A.S[i]));
+    __threadfence();
+    __syncthreads();
+    unsigned done = 0;
+    if (threadIdx.x == 0) done = atomicAdd(A.duty_done, 1u + (ask ? 65536u : 0u)) + 1u + (ask ? 65536u : 0u);
+    if (!__syncthreads_or((done & 65535u) == ctas)) return;
+    if (threadIdx.x == 0) *A.duty_done = 0;
+    __threadfence();
+    make_plan(A, __syncthreads_or(done >> 16));
 }
 
 __global__ void __launch_bounds__(512) k_sort(const __grid_constant__ BatchArgs A)
@@ -166,6 +174,7 @@ KernelSet kernel_set(int dim, int precision)
     k.topo = (void *)k_topo;
     k.sys_mark = (void *)k_sys_mark;
     k.duty = (void *)k_duty;
+    k.duty_wide = (void *)k_duty_wide;
     return k;
 }
 
