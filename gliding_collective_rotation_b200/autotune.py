@@ -30,7 +30,8 @@ import numpy as np
 # the search starts from DEFAULT
 SPACE = {
     "block_beads": (64, 128, 256),     # beads per tile = threads per CTA of the bead kernels
-    "ctas_per_sm": (0, 2, 4, 8),       # persistent CTAs per SM (0: as many as fit)
+    "ctas_per_sm": (0, 2, 4, 8),       # persistent CTAs per SM (0: as many as fit, for a context alone on the
+                                       # device; > 0: the kernels of one that shares it, see gcr_config)
     "steps_per_graph": (5, 10, 20),    # steps per captured CUDA graph
     "skin_scale": (0.67, 1.0, 1.5),    # Verlet skin relative to engine.default_skin(r_cut)
     "pair_mode": (0, 1, 2),            # pair forces: list kernel, list walk in the stages, cell-staged kernel

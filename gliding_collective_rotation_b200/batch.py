@@ -1,11 +1,13 @@
 """Many independent systems of different sizes advanced together.
 
 All systems of a ``Batch`` share one ``Engine`` (one ``libgcr`` context), so
-one captured CUDA graph of persistent kernels steps every system: the
-kernels walk a per-system tile table in device memory, each system keeps its
-own parameters, adaptive dt, step counter and Philox seed.  The bead state of
-all systems lives in a few large device tensors (per-system views), so the
-host <-> device copies of a call are single bulk transfers.
+one kernel (small batches) or one captured CUDA graph of persistent kernels
+steps every system: the kernels walk a per-system tile table in device
+memory, each system keeps its own parameters, adaptive dt, step counter and
+Philox seed.  Batches that step at the same time, each on its own stream, are
+made with ``ctas_per_sm=9``: at 0 a batch has the device to itself.  The bead
+state of all systems lives in a few large device tensors (per-system views), so
+the host <-> device copies of a call are single bulk transfers.
 
 The plain path (``PlainRunner``) advances the same systems one system per
 launch sequence, as the drop-in does; it is the baseline the batched path is

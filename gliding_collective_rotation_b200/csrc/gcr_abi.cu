@@ -1,9 +1,10 @@
 // gcr_abi.cu -- the C ABI of libgcr.so (declared in include/gcr.h).
 //
-// A context owns the scratch of many resident systems and one CUDA graph of
-// `steps_per_graph` SRK2 steps.  The graph's kernels are persistent and read
-// the system descriptors and tile tables from device memory, so admitting or
-// evicting a system (continuous batching) never re-captures the graph.
+// A context owns the scratch of many resident systems.  Small batches step in
+// one kernel; others through one CUDA graph of `steps_per_graph` steps, whose
+// kernels are persistent and read the system descriptors and tile tables from
+// device memory, so admitting or evicting a system (continuous batching) never
+// re-captures the graph.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -194,10 +195,15 @@ struct gcr_ctx {
 namespace {
 
 // list entries a thread of the list build sorts in shared memory, of which it
-// takes from the L1 cache: short lists (WCA) need few
+// takes from the L1 cache: short lists (WCA) need few.  With a build in nearly
+// every stage, us a step (B200) at 8 or 16 entries, 12 or 32, 24 or 48, 32 or 64:
+// 64 sweep systems 397, 397, 396, 401; 125k 2D LJ beads 334, 256, 250, 306; 250k
+// 3D ones 953, 899, 853, 852.
 int build_cap(int block, int list_depth) { return std::min(list_depth <= 32 ? 12 : 32, 12288 / block); }
 
 // ... and in the one-kernel steps, where the CTAs of all tiles share the SMs
+// (10,000 LJ beads, 2D and 3D, at 12, 16, 24, 32 entries 223, 217, 201, 176 and
+// 224, 222, 218, 206 us a step, again with a build in nearly every stage)
 constexpr int kTeamBuildCap = 24;
 
 // their dynamic shared memory: the list walk's buffers or the build's columns
@@ -775,9 +781,10 @@ int enqueue_run_start(gcr_ctx *c, bool one_kernel)
 }
 
 // a list build of `slot` before its next pair forces, from zeroed cell
-// counts: admission, a new descriptor (grid, cutoff, skin, exclusions), a
-// coupling change, and re-arming after a stop (a build that overflowed its
-// cells leaves their counts set)
+// counts: admission, a descriptor that changes what the lists depend on (grid,
+// list radius, skin, box, exclusions) or of a coupled system, a coupling change,
+// and re-arming after a stop (a build that overflowed its cells leaves their
+// counts set)
 int mark_rebuild(gcr_ctx *c, int slot)
 {
     const Slot &sl = c->slots[slot];
@@ -843,20 +850,22 @@ int steps_kind(const gcr_ctx *c)
 
 // Steps run in one kernel (k_steps) while every tile has a CTA of its own, of
 // those that fit at once (592 of 128 threads); a second round would wait for
-// the first between two barriers.  One step, us, by launches and in one kernel
-// (B200): 1000 beads 28, 20; 4000 30, 26; 64,000 33, 32; four sweep systems of
-// 82,000 beads, two rounds, 37, 48; FP64 1000 31, 22; 32,000 39, 30.  Coupled
-// populations and SRK4 have more barriers a step and half the limit: motors
-// 15,000 beads 94, 81, 61,000 beads 137, 153; SRK4 1500 beads 63, 37.  One CTA
-// per tile (ctas_per_sm < 0) and the cell-staged pair forces always use
-// launches.
+// the first between two barriers (82,000 beads, two rounds, 37 us a step by
+// launches and 48 so).  One step, us, by launches and in one kernel (B200): 1000
+// beads 25, 17; 4000 29, 23; 64,000 34, 29; FP64 1000 32, 20; 64,000 40, 30.
+// Coupled populations, rigid rods and SRK4 have more barriers a step and half the
+// limit: motors 15,000 beads 74, 64; 30,000 84, 81; 61,000 97, 109; rods 1000
+// beads 49, 41; 37,000 60, 60; 58,000 62, 67; SRK4 1500 beads 57, 40; 10,000 57,
+// 48.  One CTA per tile (ctas_per_sm < 0) and the cell-staged pair forces always
+// use launches.
 bool one_kernel_steps(gcr_ctx *c)
 {
     if (c->cfg.ctas_per_sm < 0 || c->cfg.pair_mode == 2) return false;
     const int kind = steps_kind(c), bb = c->cfg.block_beads;
     const int64_t tiles = (int64_t)c->h_bead_tiles.size();
     // a context told to leave room for others (ctas_per_sm) launches: cooperative
-    // kernels that do not fit together run one after another
+    // kernels that do not fit together run one after another (a step of four
+    // contexts of 64,000 beads 114 us so, 53 by launches in grids of 9 CTAs an SM)
     if (c->cfg.ctas_per_sm > 0 && tiles > 16) return false;
     // the per-system work is one CTA's: a thread a slot, or its chains of loads
     // come in turn (systems of 30 beads, by launches and in one kernel: 64 36, 30;
@@ -1321,9 +1330,8 @@ int gcr_update_desc(gcr_ctx *c, int32_t slot, const gcr_system_desc *desc)
             if (g.slots[k] != slot && c->slots[g.slots[k]].desc.L != desc->L)
                 return fail(GCR_ERR_BAD_ARG, "coupled populations share L");
     }
-    // the current grid stays while its cells cover the list radius (a new
-    // descriptor marks the system for a list build, so a grid change between
-    // calls is safe)
+    // the current grid stays while its cells cover the list radius (a change of
+    // the grid, compared below, forces a list build, so it is safe between calls)
     if (desc->calc_wca && sl.desc.calc_wca && desc->L == sl.desc.L && sl.nc >= 3 &&
         desc->L / (double)sl.nc >= desc->wca_params[3] + skin)
         nc = sl.nc;

@@ -5,7 +5,8 @@
 // correlations over chain centres (analysis.correlation_func with g_of_r,
 // Cvv, Cnn, analysis.py:203-275), for the resident systems of a context.
 // The reference computes them in Python loops, O(n_chains^2) for the
-// correlations; here one thread per chain and one per chain pair.
+// correlations; here one thread per chain, and for the pairs a thread per row
+// of a tile of 64 x 64 chains (or of a slice of its columns).
 //
 // Determinism: g(r) counts are integers; the Cvv / Cnn sums are accumulated
 // in 64-bit fixed point (2^-32 resolution per pair), so the histograms do not

@@ -153,8 +153,9 @@ constexpr int min_blocks()
 }
 
 // Registers a thread of the stage kernels.  2D mixed: 56 (9 CTAs of 128
-// threads per SM).  With the pair walk in the stage the sweep's two stages
-// take 267 + 216 us so, 283 + 222 at 48 (spills) and about 3% more at 64.
+// threads per SM; 72 and 64 bytes of spill stores in the two SRK2 stages that
+// walk the lists, up to 84 in SRK4's).  The sweep's two stages take 267 + 216 us
+// so, 283 + 222 at 48, where more is spilled, and about 3% more at 64.
 #ifndef GCR_STAGE2D_REGS
 #define GCR_STAGE2D_REGS 56
 #endif

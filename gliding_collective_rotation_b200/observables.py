@@ -6,8 +6,8 @@
   angle of ``output_methods.calc_avg_phi_chain`` (output_methods.py:492-510)
   with 1- and 2-fold symmetry; on the GPU (``gcr_chain_frames``).
 * ``pair_correlation``: ``analysis.g_of_r``, ``analysis.Cvv`` and
-  ``analysis.Cnn`` (analysis.py:203-275) over the chain centres, one GPU
-  thread per chain pair (``gcr_pair_correlation``); 2D.
+  ``analysis.Cnn`` (analysis.py:203-275) over the chain centres, a GPU
+  thread per row of a tile of chain pairs (``gcr_pair_correlation``); 2D.
 * ``order_parameters``: P, S and the director angle
   (analysis.py:294-328, ``gcr_order_params``).
 * ``rotation_rate`` and ``remove_outliers``: the collective rotation rate of

@@ -90,7 +90,16 @@ typedef struct {
     int32_t block_beads;      /* threads per CTA of bead kernels (64..512) */
     int32_t block_cells;      /* threads per CTA of the cell kernel (64..512) */
     int32_t steps_per_graph;  /* steps per captured CUDA graph (1..64); gcr_run takes a multiple of it */
-    int32_t ctas_per_sm;      /* persistent CTAs per SM (0 = from occupancy, <0 = one CTA per tile) */
+    int32_t ctas_per_sm;      /* persistent CTAs per SM of the step kernels (0 = as many as fit, <0 = one
+                                 CTA per tile), and whether the context shares the device.
+                                 0: alone.  A small batch steps in one kernel, a cooperative launch
+                                 beyond 16 tiles of block_beads; 2D mixed stages walk the lists
+                                 themselves.  Contexts that step at the same time set it above 0
+                                 (9 measured best): cooperative kernels that do not fit together run
+                                 one after another.
+                                 > 0: one kernel up to 16 tiles only (one cluster), else launches with
+                                 a pair kernel, whose grids the other contexts' can share the SMs with.
+                                 < 0: always launches.  The results are the same bits */
     int32_t list_depth;       /* neighbour-list slots per bead, 4..1024 (0 = 32 in 2D, 96 in 3D) */
     int32_t srk_order;        /* config.SRK_order: 2 (0 = 2) or 4 (SRK.py:144-215, 296-321) */
     int32_t pair_mode;        /* pair forces of SRK2 contexts while no system is coupled to another
@@ -256,8 +265,10 @@ GCR_API int gcr_where_active(gcr_ctx *ctx, int32_t slot, int32_t *dst);
 
 /* ---- stepping --------------------------------------------------------- */
 /* Advance every armed system until its limits are reached or `max_steps`
- * steps have been launched, through captured CUDA graphs of
- * steps_per_graph steps.  `sync_every` graphs between checks of whether any
+ * steps have been launched: small batches in one kernel for up to 512
+ * steps, others through captured CUDA graphs of steps_per_graph steps; a
+ * multiple of steps_per_graph either way.  `sync_every` graphs (or as many
+ * steps in one kernel) between checks of whether any
  * system is still running (0: never check; run exactly ceil(max_steps /
  * steps_per_graph) graphs).  Asynchronous on the context stream unless a
  * check is made. */
