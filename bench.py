@@ -374,8 +374,9 @@ def run_gpu(args):
     from gliding_collective_rotation_b200.batch import Batch, PlainRunner
     from gliding_collective_rotation_b200.engine import default_skin
     from gliding_collective_rotation_b200._lib import (FLAG_CELL_OVERFLOW, FLAG_LIST_CORRUPT, FLAG_LIST_OVERFLOW,
-                                                       FLAG_NONFINITE)
-    FLAG_FATAL = FLAG_CELL_OVERFLOW | FLAG_NONFINITE | FLAG_LIST_CORRUPT | FLAG_LIST_OVERFLOW
+                                                       FLAG_NONFINITE, FLAG_WAIT_EXPIRED)
+    FLAG_FATAL = (FLAG_CELL_OVERFLOW | FLAG_NONFINITE | FLAG_LIST_CORRUPT | FLAG_LIST_OVERFLOW
+                  | FLAG_WAIT_EXPIRED)
     regrows = 0
 
     world = int(os.environ.get("WORLD_SIZE", "1"))
